@@ -17,6 +17,7 @@
 #include "../../include/fecl_b200.h"
 #include "device/kernels.hpp"
 #include "host/codes.hpp"
+#include "host/encode_plan.hpp"
 #include "host/ldpc_plan.hpp"
 #include "host/puncture.hpp"
 
@@ -128,7 +129,7 @@ struct fecl_codec_s {
   DeviceBuffer crc_tab;   // CRC syndrome table of the turbo decoder's CRC stop
   // The CRC stop's syndrome table on the device, or null when the decoder has none.
   const uint32_t* crc_table() const { return (kind == 1 && turbo->decoder().crc) ? crc_tab.as<uint32_t>() : nullptr; }
-  DeviceBuffer enc[8];  // LDPC generator pieces (DC, A, B, T as CSR) for the device encoder
+  DeviceBuffer enc[8];  // the device encoder's tables (ltab)
   fecl::LdpcEncodeTables ltab;
   fecl::TurboDeviceCode tdev;
   // workspace
@@ -196,27 +197,59 @@ struct fecl_codec_s {
     ldev.col_idx = col_idx.as<uint32_t>();
     ldev.col_ptr = col_ptr.as<uint32_t>();
     ldev.col_edges = col_edges.as<uint32_t>();
-    const fecl::Csr* parts[4] = {&ldpc->gen_dc(), &ldpc->gen_a(), &ldpc->gen_b(), &ldpc->gen_t()};
-    for (int i = 0; i < 4; ++i) {
-      enc[2 * i].upload(parts[i]->row_ptr);
-      enc[2 * i + 1].upload(parts[i]->col_idx);
-    }
+    upload_ldpc_encoder();
+    upload_ldpc_options();
+  }
+
+  void upload_ldpc_encoder() {
+    ltab = fecl::LdpcEncodeTables{};
     ltab.K = int32_t(ldpc->msg_size());
-    ltab.N = int32_t(H.cols);
+    ltab.N = int32_t(ldpc->parity_size());
     ltab.gap = int32_t(ldpc->gen_dc().rows);
-    ltab.dc_rows = int32_t(ldpc->gen_dc().rows);
+    enc[0].upload(ldpc->gen_dc().row_ptr);
+    enc[1].upload(ldpc->gen_dc().col_idx);
+    ltab.dc_rows = ltab.gap;
+    ltab.dc_ptr = enc[0].as<uint32_t>();
+    ltab.dc_idx = enc[1].as<uint32_t>();
+    const fecl::LdpcEncodePlan plan = fecl::build_ldpc_encode_plan(*ldpc, uint32_t(smem_optin) - 1024);
+    if (plan.ok) {
+      ltab.bytes = plan.bytes;
+      ltab.zero_at = plan.zero_at;
+      ltab.off_gap = plan.off_gap;
+      ltab.off_t = plan.off_t;
+      ltab.rows = int32_t(ldpc->gen_a().rows);
+      ltab.chain = plan.chain ? 1 : 0;
+      enc[2].upload(plan.row_ptr);
+      enc[3].upload(plan.row_idx);
+      ltab.row_ptr = enc[2].as<uint32_t>();
+      ltab.row_idx = enc[3].as<uint32_t>();
+      if (!plan.chain) {
+        ltab.levels = int32_t(plan.level_ptr.size()) - 1;
+        enc[4].upload(plan.level_ptr);
+        enc[5].upload(plan.level_rows);
+        enc[6].upload(plan.src_ptr);
+        enc[7].upload(plan.src_idx);
+        ltab.level_ptr = enc[4].as<uint32_t>();
+        ltab.level_rows = enc[5].as<uint32_t>();
+        ltab.src_ptr = enc[6].as<uint32_t>();
+        ltab.src_idx = enc[7].as<uint32_t>();
+      }
+      return;
+    }
+    const fecl::Csr* parts[3] = {&ldpc->gen_a(), &ldpc->gen_b(), &ldpc->gen_t()};
+    for (int i = 0; i < 3; ++i) {
+      enc[2 * i + 2].upload(parts[i]->row_ptr);
+      enc[2 * i + 3].upload(parts[i]->col_idx);
+    }
     ltab.a_rows = int32_t(ldpc->gen_a().rows);
     ltab.b_rows = int32_t(ldpc->gen_b().rows);
     ltab.t_rows = int32_t(ldpc->gen_t().rows);
-    ltab.dc_ptr = enc[0].as<uint32_t>();
-    ltab.dc_idx = enc[1].as<uint32_t>();
     ltab.a_ptr = enc[2].as<uint32_t>();
     ltab.a_idx = enc[3].as<uint32_t>();
     ltab.b_ptr = enc[4].as<uint32_t>();
     ltab.b_idx = enc[5].as<uint32_t>();
     ltab.t_ptr = enc[6].as<uint32_t>();
     ltab.t_idx = enc[7].as<uint32_t>();
-    upload_ldpc_options();
   }
 
   void upload_ldpc_options() {

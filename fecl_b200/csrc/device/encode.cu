@@ -1,7 +1,6 @@
 // Device encoders and the BPSK/AWGN channel.
 //
-// The encoders run the reference's encoding steps with one thread per frame (per
-// frame and constituent for turbo codes), so their output is bit-exact with
+// The encoders run the reference's encoding steps, so their output is bit-exact with
 // LdpcCode::encode / TurboCode::encode and the reference they restate:
 //   LDPC  systematic copy, then the sparse XOR steps of Ldpc::Structure::encode
 //         (src/detail/Ldpc.cpp:180-209): gap parity from the message (DC), the
@@ -24,7 +23,203 @@
 namespace fecl {
 namespace {
 
-__global__ void ldpc_encode_kernel(LdpcEncodeTables t, const uint8_t* msg, uint8_t* parity, int64_t nframes) {
+// LDPC encoding, a CTA per `per` (at most 8) frames with the whole code word in shared
+// memory: byte i holds bit i of the CTA's frames, frame f in its bit f, so one byte xor
+// serves all of them and the code's tables are read once per CTA.  Bound by the gathers
+// of the T-part rows (one shared byte per edge and CTA); a thread per row, its entries
+// interleaved over the 32 rows of a warp so that their loads are contiguous.  The
+// accumulator of the DVB-S2 codes is a prefix xor: each thread folds an odd number of
+// words (so that the threads' strides fall into different banks), the threads' totals
+// are scanned over the block, and the words are written back with their carries.  Other
+// T parts are solved level by level.  V: bytes per access of the caller's buffers.
+// 512 DVB-S2 normal r=1/2 frames: 35 us a call (1.4 TB/s of bits in and out) against
+// 44.6 ms with a thread per frame, whose single chain of dependent loads left the GPU
+// idle; 79 us before a warp's entry lines were streamed.
+template <int V>
+struct EncodeVec;
+template <>
+struct EncodeVec<16> {
+  uint4 v;
+};
+template <>
+struct EncodeVec<8> {
+  uint2 v;
+};
+template <>
+struct EncodeVec<4> {
+  uint32_t v;
+};
+template <>
+struct EncodeVec<1> {
+  uint8_t v;
+};
+
+constexpr int kEncodeFrames = 8;  // frames per CTA at most: the bits of a byte
+
+// Bit f of every byte, and the frames' bits folded into one byte each.
+__device__ __forceinline__ uint32_t bit_of(uint32_t w, int f) { return (w >> f) & 0x01010101u; }
+__device__ __forceinline__ uint4 bit_of(uint4 w, int f) {
+  return make_uint4(bit_of(w.x, f), bit_of(w.y, f), bit_of(w.z, f), bit_of(w.w, f));
+}
+__device__ __forceinline__ uint2 bit_of(uint2 w, int f) { return make_uint2(bit_of(w.x, f), bit_of(w.y, f)); }
+__device__ __forceinline__ uint8_t bit_of(uint8_t w, int f) { return uint8_t((w >> f) & 1); }
+__device__ __forceinline__ void fold(uint32_t& a, uint32_t w, int f) { a |= w << f; }
+__device__ __forceinline__ void fold(uint4& a, uint4 w, int f) {
+  fold(a.x, w.x, f);
+  fold(a.y, w.y, f);
+  fold(a.z, w.z, f);
+  fold(a.w, w.w, f);
+}
+__device__ __forceinline__ void fold(uint2& a, uint2 w, int f) {
+  fold(a.x, w.x, f);
+  fold(a.y, w.y, f);
+}
+__device__ __forceinline__ void fold(uint8_t& a, uint8_t w, int f) { a = uint8_t(a | (w << f)); }
+
+// Writes bits [0, n) of s to position `at` of each of the nf frames' code words.
+template <int V>
+__device__ __forceinline__ void put_bits(const uint8_t* s, int n, uint8_t* parity, int64_t N, int64_t at, int nf) {
+  using T = decltype(EncodeVec<V>::v);
+  for (int i = int(threadIdx.x) * V; i < n; i += int(blockDim.x) * V) {
+    const T w = *reinterpret_cast<const T*>(s + i);
+#pragma unroll
+    for (int f = 0; f < kEncodeFrames; ++f)
+      if (f < nf) *reinterpret_cast<T*>(parity + f * N + at + i) = bit_of(w, f);
+  }
+}
+
+template <int V>
+__global__ void __launch_bounds__(1024) ldpc_encode_kernel(LdpcEncodeTables t, const uint8_t* msg, uint8_t* parity,
+                                                           int64_t nframes, int per) {
+  using T = decltype(EncodeVec<V>::v);
+  extern __shared__ __align__(16) uint8_t s[];
+  __shared__ uint32_t part[32];
+  const int tid = int(threadIdx.x), threads = int(blockDim.x), lane = tid & 31, warp = tid >> 5, warps = threads >> 5;
+  const int64_t f0 = int64_t(blockIdx.x) * per;
+  const int nf = int(nframes - f0 < per ? nframes - f0 : per);
+  const uint8_t* m = msg + f0 * t.K;
+  uint8_t* c = parity + f0 * t.N;
+
+  // the message: copied to the code words and folded into shared memory
+  for (int i = tid * V; i < t.K; i += threads * V) {
+    T w[kEncodeFrames];
+#pragma unroll
+    for (int f = 0; f < kEncodeFrames; ++f)
+      if (f < nf) w[f] = bit_of(*reinterpret_cast<const T*>(m + int64_t(f) * t.K + i), 0);
+    T acc = {};
+#pragma unroll
+    for (int f = 0; f < kEncodeFrames; ++f)
+      if (f < nf) {
+        *reinterpret_cast<T*>(c + int64_t(f) * t.N + i) = w[f];
+        fold(acc, w[f], f);
+      }
+    *reinterpret_cast<T*>(s + i) = acc;
+  }
+  if (tid == 0) s[t.zero_at] = 0;
+  __syncthreads();
+
+  // gap parity from the message: dense rows, a warp each
+  uint8_t* gap = s + t.off_gap;
+  for (int r = warp; r < t.gap; r += warps) {
+    uint32_t v = 0;
+    for (uint32_t e = t.dc_ptr[r] + lane; e < t.dc_ptr[r + 1]; e += 32) v ^= s[t.dc_idx[e]];
+    v = __reduce_xor_sync(0xffffffffu, v);
+    if (lane == 0) gap[r] = uint8_t(v);
+  }
+  if (t.gap) __syncthreads();
+
+  // T-part rows: the message (A) and gap (B) columns.  A warp takes a run of blocks and
+  // streams their entry lines, kAhead lines loaded while the kAhead before are gathered;
+  // lane l holds the end of the run's block l.
+  uint8_t* p = s + t.off_t;
+  constexpr int kAhead = 8;
+  const int blocks = (t.rows + 31) / 32, run = (blocks + warps - 1) / warps;
+  const int b_end = min(blocks, (warp + 1) * run);
+  for (int b = warp * run; b < b_end; b += 32) {
+    const int nb = min(32, b_end - b);
+    const uint32_t ends = t.row_ptr[min(b + lane + 1, blocks)];
+    uint32_t e = t.row_ptr[b];
+    const uint32_t last = __shfl_sync(0xffffffffu, ends, nb - 1);
+    uint32_t next[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) next[j] = e + 32 * j < last ? __ldg(t.row_idx + e + 32 * j + lane) : t.zero_at;
+    uint32_t v = 0, end = __shfl_sync(0xffffffffu, ends, 0);
+    int cur = 0;
+    for (; e < last; e += 32 * kAhead) {
+      uint32_t idx[kAhead];
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        idx[j] = next[j];
+        const uint32_t a = e + 32 * (kAhead + j);
+        next[j] = a < last ? __ldg(t.row_idx + a + lane) : t.zero_at;
+      }
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        while (cur < nb && end == e + 32 * j) {  // block cur is complete (or has no entries)
+          const int r = (b + cur) * 32 + lane;
+          if (r < t.rows) p[r] = uint8_t(v);
+          v = 0;
+          if (++cur < nb) end = __shfl_sync(0xffffffffu, ends, cur);
+        }
+        v ^= s[idx[j]];
+      }
+    }
+    for (; cur < nb; ++cur) {  // the last block with entries, and empty ones after it
+      const int r = (b + cur) * 32 + lane;
+      if (r < t.rows) p[r] = uint8_t(v);
+      v = 0;
+    }
+  }
+  __syncthreads();
+
+  // back substitution through T
+  if (t.chain) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(p);
+    const int words = (t.rows + 3) / 4;
+    if (tid < words * 4 - t.rows) p[t.rows + tid] = 0;
+    const int each = ((words + threads - 1) / threads) | 1;
+    const int w0 = tid * each, w1 = min(words, w0 + each);
+    __syncthreads();
+    uint32_t x = 0;
+    for (int i = w0; i < w1; ++i) x ^= w[i];
+    x ^= x >> 16;
+    x = (x ^ (x >> 8)) & 0xffu;
+    uint32_t upto = x;  // inclusive scan over the warp
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto ^= y;
+    }
+    if (lane == 31) part[warp] = upto;
+    __syncthreads();
+    uint32_t carry = upto ^ x;
+    for (int q = 0; q < warp; ++q) carry ^= part[q];
+    for (int i = w0; i < w1; ++i) {
+      uint32_t v = w[i];
+      v ^= v << 8;
+      v ^= v << 16;
+      v ^= carry * 0x01010101u;
+      w[i] = v;
+      carry = v >> 24;
+    }
+    __syncthreads();
+  } else {
+    for (int l = 0; l < t.levels; ++l) {
+      for (uint32_t q = t.level_ptr[l] + tid; q < t.level_ptr[l + 1]; q += threads) {
+        const uint32_t r = t.level_rows[q];
+        uint32_t v = p[r];
+        for (uint32_t e = t.src_ptr[q]; e < t.src_ptr[q + 1]; ++e) v ^= p[t.src_idx[e]];
+        p[r] = uint8_t(v);
+      }
+      __syncthreads();
+    }
+  }
+  put_bits<V>(gap, t.gap, c, t.N, t.K, nf);
+  put_bits<V>(p, t.rows, c, t.N, int64_t(t.K) + t.gap, nf);
+}
+
+// The same steps with one thread per frame, for code words beyond shared memory.
+__global__ void ldpc_encode_long_kernel(LdpcEncodeTables t, const uint8_t* msg, uint8_t* parity, int64_t nframes) {
   const int64_t f = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (f >= nframes) return;
   const uint8_t* m = msg + f * t.K;
@@ -166,8 +361,34 @@ unsigned blocks_for(int64_t threads, int per_block) {
 cudaError_t launch_ldpc_encode(const LdpcEncodeTables& t, const uint8_t* msg, uint8_t* parity, int64_t nframes,
                                cudaStream_t s) {
   if (nframes <= 0) return cudaSuccess;
-  ldpc_encode_kernel<<<blocks_for(nframes, 64), 64, 0, s>>>(t, msg, parity, nframes);
-  return cudaGetLastError();
+  if (!t.bytes) {
+    ldpc_encode_long_kernel<<<blocks_for(nframes, 64), 64, 0, s>>>(t, msg, parity, nframes);
+    return cudaGetLastError();
+  }
+  // Frames per CTA: as few as let one round of CTAs, one per SM, take the batch (the row
+  // gathers cost the same for 1 and for 8 frames), at most the 8 bits of a byte.
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  int64_t per = (nframes + sms - 1) / sms;
+  if (per > kEncodeFrames) per = kEncodeFrames;
+  const int64_t blocks = (nframes + per - 1) / per;
+  if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+  const int threads = t.N >= 8192 ? 1024 : 256;
+  // the widest access that divides the parts of a code word and both buffers' alignment
+  const uintptr_t parts = uintptr_t(t.K) | uintptr_t(t.N) | uintptr_t(t.gap) | reinterpret_cast<uintptr_t>(msg) |
+                          reinterpret_cast<uintptr_t>(parity);
+  auto run = [&](auto kern) -> cudaError_t {
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(t.bytes));
+    if (err != cudaSuccess) return err;
+    kern<<<unsigned(blocks), threads, t.bytes, s>>>(t, msg, parity, nframes, int(per));
+    return cudaGetLastError();
+  };
+  if (parts % 16 == 0) return run(ldpc_encode_kernel<16>);
+  if (parts % 8 == 0) return run(ldpc_encode_kernel<8>);
+  if (parts % 4 == 0) return run(ldpc_encode_kernel<4>);
+  return run(ldpc_encode_kernel<1>);
 }
 
 cudaError_t launch_turbo_encode(const TurboDeviceCode& code, const uint8_t* msg, uint8_t* parity, int64_t nframes,

@@ -349,6 +349,12 @@ struct LdpcEncodeTables {
   const uint32_t *a_ptr = nullptr, *a_idx = nullptr;
   const uint32_t *b_ptr = nullptr, *b_idx = nullptr;
   const uint32_t *t_ptr = nullptr, *t_idx = nullptr;
+  // the shared-memory encoder's tables (host/encode_plan.hpp); bytes == 0: the code takes
+  // the thread-per-frame encoder, which alone reads the A, B and T pieces above
+  uint32_t bytes = 0, zero_at = 0, off_gap = 0, off_t = 0;
+  int32_t rows = 0, chain = 0, levels = 0;
+  const uint32_t *row_ptr = nullptr, *row_idx = nullptr;
+  const uint32_t *level_ptr = nullptr, *level_rows = nullptr, *src_ptr = nullptr, *src_idx = nullptr;
 };
 cudaError_t launch_ldpc_encode(const LdpcEncodeTables& t, const uint8_t* msg, uint8_t* parity, int64_t nframes,
                                cudaStream_t s);

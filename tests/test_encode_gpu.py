@@ -87,3 +87,27 @@ def test_device_inputs_decode_end_to_end():
         assert np.array_equal(bits.cpu().numpy(), code.decode(llr.cpu().numpy()))
         errors = (bits != msg).view(n, K).any(dim=1).sum().item()
         assert errors == 0, (K, errors)
+
+
+@pytest.mark.parametrize("frames", [1, 149, 1185])
+@pytest.mark.parametrize("code", ["gallager-2048", "gallager-256", "short-1/2", "normal-9/10"])
+def test_ldpc_encoder_frames_per_cta_and_alignment(code, frames):
+    """1, 2 and 8 (with a partial last CTA) frames per CTA; accumulator and levelled T
+    parts, with and without a gap; buffers at odd addresses.  Bits: equal."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    if code.startswith("gallager"):
+        n = int(code.split("-")[1])
+        H = F.Ldpc.Gallager.matrix(n, 3, 5 if n == 2048 else 6, 0 if n == 2048 else 1)
+        c = F.Ldpc(F.Ldpc.EncoderOptions(H), F.Ldpc.DecoderOptions())
+    else:
+        c = _ldpc(*((16200, (1, 2)) if code == "short-1/2" else (64800, (9, 10))))
+    if c.paritySize() > 20000 and frames > 149:
+        frames = 297  # 3 per CTA: the host encoder's time
+    msg = ch.random_bits(frames * c.msgSize(), 62)
+    want = torch.from_numpy(c.encode(msg)).cuda()
+    for offset in (0, 1, 4):
+        buf = torch.zeros(offset + msg.size, dtype=torch.uint8, device="cuda")
+        buf[offset:] = torch.from_numpy(msg).cuda() | 0xFE if offset == 1 else torch.from_numpy(msg).cuda()
+        assert torch.equal(c.encode(buf[offset:]), want), offset
