@@ -267,6 +267,30 @@ struct fecl_codec_s {
     ldev.fixed_iterations = d.fixed_iterations;
   }
 
+  // A constituent's tables in one allocation: next_state | output | predecessors | perm,
+  // each from a multiple of 4 entries (perm is read in vectors).
+  void upload_trellis(const fecl::Trellis& t, const std::vector<uint32_t>& perm, fecl::TurboDeviceConstituent& k) {
+    std::vector<uint32_t> all;
+    size_t at[4];
+    const std::vector<uint32_t> pred = t.predecessors();
+    const std::vector<uint32_t>* parts[4] = {&t.next_state, &t.output, &pred, &perm};
+    for (int i = 0; i < 4; ++i) {
+      all.resize((all.size() + 3) / 4 * 4, 0);
+      at[i] = all.size();
+      all.insert(all.end(), parts[i]->begin(), parts[i]->end());
+    }
+    tables.emplace_back(new DeviceBuffer);
+    tables.back()->upload(all);
+    const uint32_t* base = tables.back()->as<uint32_t>();
+    k.next_state = base + at[0];
+    k.output = base + at[1];
+    k.pred = pred.empty() ? nullptr : base + at[2];
+    k.pred_paired = t.state_count == 64 && t.input_count == 2 && !pred.empty();
+    for (size_t i = 0; i < pred.size() && k.pred_paired; i += 2)
+      if ((pred[i] & 1) || (pred[i + 1] & 0xff) != (pred[i] & 0xff) + 1) k.pred_paired = 0;
+    k.perm = base + at[3];
+  }
+
   void upload_turbo() {
     const auto& cs = turbo->constituents();
     if (cs.size() > size_t(fecl::kMaxConstituents)) fail(FECL_EUNSUPPORTED, "too many constituents for the device decoder");
@@ -296,14 +320,7 @@ struct fecl_codec_s {
       // interleavers are padded with zeros so that 8-entry vector loads never leave them
       std::vector<uint32_t> padded_perm(c.perm);
       padded_perm.resize(c.perm.size() + 16, 0);
-      for (const std::vector<uint32_t>* v : {&c.trellis.next_state, &c.trellis.output,
-                                             static_cast<const std::vector<uint32_t>*>(&padded_perm)}) {
-        tables.emplace_back(new DeviceBuffer);
-        tables.back()->upload(*v);
-      }
-      k.next_state = tables[tables.size() - 3]->as<uint32_t>();
-      k.output = tables[tables.size() - 2]->as<uint32_t>();
-      k.perm = tables[tables.size() - 1]->as<uint32_t>();
+      upload_trellis(c.trellis, padded_perm, k);
       tdev.max_steps = std::max(tdev.max_steps, int32_t(c.length + c.tail));
       tdev.max_states = std::max(tdev.max_states, int32_t(c.trellis.state_count));
     }
@@ -317,11 +334,7 @@ struct fecl_codec_s {
     tables.clear();
     std::vector<uint32_t> padded_perm(c.perm);
     padded_perm.resize(c.perm.size() + 16, 0);
-    for (const std::vector<uint32_t>* v : {&c.trellis.next_state, &c.trellis.output,
-                                           static_cast<const std::vector<uint32_t>*>(&padded_perm)}) {
-      tables.emplace_back(new DeviceBuffer);
-      tables.back()->upload(*v);
-    }
+    upload_trellis(c.trellis, padded_perm, cdev);
     cdev.state_count = int32_t(c.trellis.state_count);
     cdev.input_count = int32_t(c.trellis.input_count);
     cdev.input_size = int32_t(c.trellis.input_size);
@@ -333,9 +346,6 @@ struct fecl_codec_s {
     cdev.syst_size = int32_t(c.syst_size());
     cdev.syst_tail_size = int32_t(c.syst_tail_size());
     cdev.parity_size = int32_t(c.parity_size());
-    cdev.next_state = tables[0]->as<uint32_t>();
-    cdev.output = tables[1]->as<uint32_t>();
-    cdev.perm = tables[2]->as<uint32_t>();
   }
 
   void upload_turbo_options() {

@@ -184,6 +184,12 @@ struct TurboDeviceConstituent {
   const uint32_t* next_state;  // [state_count * input_count]
   const uint32_t* output;
   const uint32_t* perm;        // [msg_size]
+  // Where every state has input_count predecessors: entry [state * input_count + i] is
+  // state | input << 8 | output << 16 of the i-th branch into the state, in (state,
+  // input) order; null otherwise.
+  const uint32_t* pred = nullptr;
+  // 64 states, 2 inputs, and states 2 m and 2 m + 1, for one m, the two predecessors of every state
+  int32_t pred_paired = 0;
 };
 
 struct TurboDeviceCode {

@@ -442,6 +442,18 @@ Trellis Trellis::from_generators(const std::vector<uint32_t>& cl, const std::vec
   return t;
 }
 
+std::vector<uint32_t> Trellis::predecessors() const {
+  if (state_count > 256 || input_count > 256 || output_size > 16) return {};
+  std::vector<uint32_t> table(size_t(state_count) * input_count), filled(state_count, 0);
+  for (uint32_t s = 0; s < state_count; ++s)
+    for (uint32_t u = 0; u < input_count; ++u) {
+      const uint32_t n = next_state[s * input_count + u];
+      if (filled[n] == input_count) return {};
+      table[size_t(n) * input_count + filled[n]++] = s | (u << 8) | (output[s * input_count + u] << 16);
+    }
+  return table;  // state_count * input_count branches, none left over: every state has its share
+}
+
 Trellis Trellis::from_tables(uint32_t state_count, uint32_t input_count, uint32_t output_size,
                              const uint32_t* next_state, const uint32_t* output) {
   Trellis t;

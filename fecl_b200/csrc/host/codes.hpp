@@ -105,6 +105,11 @@ struct Trellis {
   // Trellis given by tables (state/output counts must be powers of two).
   static Trellis from_tables(uint32_t state_count, uint32_t input_count, uint32_t output_size,
                              const uint32_t* next_state, const uint32_t* output);
+
+  // The branches into each state, input_count of them, in (state, input) order: entry
+  // [n * input_count + i] is state | input << 8 | output << 16.  Empty where a state has
+  // another number of branches or a field does not fit.
+  std::vector<uint32_t> predecessors() const;
 };
 
 struct Constituent {
