@@ -386,6 +386,7 @@ int fecl_batch_create(const fecl_batch_job* jobs, uint32_t njobs, int32_t flags,
         p.counter = reinterpret_cast<int32_t*>(base + cnt_off[kv.first]);
         p.max_K = tmax_k[kv.first];
         p.algorithm = kv.first;
+        p.whole = std::all_of(kv.second.begin(), kv.second.end(), [](const fecl::TurboLteBatchFrame& t) { return t.K % 8 == 0; });
         cuda_check(fecl::launch_turbo_lte_batch(p, b->cap), "turbo batch launch");
         plan << "turbo LTE mixed-K x" << kv.second.size() << " (alg " << kv.first << ", max K " << p.max_K << ")\n";
       }

@@ -266,7 +266,8 @@ struct TurboLteParams {
   void* state_out = nullptr;       // [nframes][2 (K + 3)]
   int32_t out_dtype = 1;
   // filled by the launcher
-  int32_t Kp = 0, Tp = 0, seg_len = 0;
+  int32_t Kp = 0, Tp = 0, seg_len = 0, segments = 0, seg_stride = 0, slots = 0;
+  uint4* perm_pos = nullptr;  // [slots] interleaved positions
   int64_t frame0 = 0;  // frame of the launch's first CTA
   int64_t frame_stride = 0;
   float* ck = nullptr;
@@ -297,10 +298,11 @@ struct TurboLteBatchParams {
   int32_t algorithm = 2;       // one algorithm per launch
   int32_t train = -1;          // training steps (-1: default)
   int32_t ctas = 0;            // persistent CTAs (0: as many as are resident at once)
+  int32_t whole = 0;           // every frame's K is a multiple of 8
   unsigned long long* stats = nullptr;
 };
 size_t turbo_lte_frame_floats(int K);
-int turbo_lte_batch_max_ctas(int max_K, int algorithm);
+int turbo_lte_batch_max_ctas(int max_K, int algorithm, bool whole);
 cudaError_t launch_turbo_lte_batch(const TurboLteBatchParams& p, cudaStream_t s);
 
 // ---- convolutional codec (conv.cu, turbo_generic.cu) -----------------------

@@ -39,13 +39,12 @@
 // and it removes the eight-way maximum and the subtractions from seven steps of
 // eight.  Global loads of the next chunk are issued one chunk ahead.
 //
-// Inputs are first converted into a padded FP32 scratch layout so that every
-// block load is 16-byte aligned.
+// Inputs are first converted into an FP32 scratch layout in which the walkers of a warp
+// read neighbouring 16-byte pieces (LteMap).
 #include <math.h>
 
-#include <map>
-#include <mutex>
-#include <utility>
+#include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.hpp"
@@ -70,7 +69,13 @@ constexpr Tol kDecodeTol = {1e-3f, 1e-5f};
 constexpr Tol kSoftTol = {1e-6f, 1e-6f};
 constexpr int kDefaultSegs = 64;
 
-__constant__ LinearLut c_lut;
+// The Linear table as (slope, value) pairs of its intervals, and a last pair of zeros for
+// everything from 3.5 on; copied to shared memory by the kernels that look it up.
+struct LinearPairs {
+  float2 v[8];
+};
+__constant__ LinearPairs c_lut;
+__shared__ float2 s_lut[8];
 
 // The LTE RSC, Trellis({4}, {{015}}, {013}) (src/Trellis.cpp:76-143): with state bits
 // s0 s1 s2, the feedback bit is u ^ s0 ^ s1, the next state shifts it in at the top
@@ -79,11 +84,19 @@ __constant__ LinearLut c_lut;
 __host__ __device__ constexpr int lte_next(int s, int u) { return (s >> 1) | (((u ^ s ^ (s >> 1)) & 1) << 2); }
 __host__ __device__ constexpr int lte_out(int s, int u) { return (u ^ (s >> 1) ^ (s >> 2)) & 1; }
 
+// The recursive log-sums (src/detail/LlrMetrics.h:88-121): max, or max plus the table's value
+// at |a - b| (nothing where a == b).  The lookup is lut_log1pexpm's, without branches or
+// conversions: floor(x) for x in [0, 7] is the low bits of x + 2^23 rounded toward zero,
+// and one 8-byte shared load fetches the interval.  Lanes look up different
+// entries, which constant memory serves one address at a time.
 template <int ALG>
 __device__ __forceinline__ float lsum(float a, float b) {
   if (ALG == kApproximate) return fmaxf(a, b);
-  if (a == b) return a;
-  return fmaxf(a, b) + lut_log1pexpm(c_lut, fabsf(a - b));
+  const float x = fminf(2.0f * fabsf(a - b), 7.0f);  // 7 also for two equal infinities
+  const float up = __fadd_rz(x, 8388608.0f);
+  const float2 e = s_lut[__float_as_uint(up) & 7u];
+  const float r = fmaxf(a, b) + __fmaf_rn(e.x, x - (up - 8388608.0f), e.y);
+  return a == b ? a : r;
 }
 
 // max(a, b, c) in one instruction (the three-input form of max.f32, sm_100): the same
@@ -321,13 +334,30 @@ __device__ __forceinline__ float par_step(const float a[8], const float b[8], co
   }
 }
 
+// Where a frame's values lie.  A frame is cut into S segments of Lc chunks of 8 steps; the
+// walkers of a warp stand at the same chunk k of neighbouring segments w, so every staged
+// array holds its chunks by k and then by w: chunk c = w Lc + k at slot k Sp + w, as two
+// planes of 4 floats per slot.  A warp's load of one plane is then contiguous (with the
+// chunks in time order it touched one line per lane, and the L1 pipe, at 73 % of its
+// peak, bound the kernel).  The exchange arrays in shared memory hold step t at
+// (t mod 8) nblk + t / 8: neighbouring chunks fall into neighbouring banks, and so do, for
+// an odd number of chunks per segment, the interleaved positions, since a QPP interleaver
+// maps steps that differ by a multiple of 8 to positions that do.
+struct LteMap {
+  int Lc, S, Sp, slots, nblk;
+  __device__ __forceinline__ int slot_of(int c) const { return (c % Lc) * Sp + c / Lc; }
+  __device__ __forceinline__ int pos(int t) const { return (t & 7) * nblk + (t >> 3); }
+};
+
 struct Frame {
-  const float* Ls;   // [Tp] systematic L-values, zero past K
-  const float* Lp0;  // [Tp]  parity (with tail parity) of constituent 0
-  const float* Lp1;  // [Tp]
-  const float* ts;   // [8]   tail systematic of constituent 0 (3) then 1 (3)
-  float* cka;        // [nblk + 1][8]
-  float* ckb;        // [nblk + 1][8]
+  LteMap m;
+  const float* Ls;    // [2][slots][4] systematic L-values, zero past K
+  const float* Lp0;   // [2][slots][4] parity (with tail parity) of constituent 0
+  const float* Lp1;   // [2][slots][4]
+  const float* ts;    // [8]  tail systematic of constituent 0 (3) then 1 (3)
+  const uint4* perm;  // [slots] position of each step's interleaved index, 16 bits each
+  float* cka;         // [2][slots][4] forward metrics before each chunk
+  float* ckb;         // [2][slots][4] backward metrics before each chunk (chunk nblk: the end)
 };
 
 // A segment's boundary vectors: a forward segment's start (after training) is its
@@ -335,31 +365,35 @@ struct Frame {
 // checkpoint arrays (global memory); the other two are kept here.
 template <int SEGS>
 struct Shared {
-  float bwd_start[SEGS][8];  // backward segment w's metrics at its end a1 after training
-  float fwd_end[SEGS][8];    // forward segment w's metrics at a1
-  float flat[8];             // training start: all states equal
-  float term[8];             // trellis termination: state 0
+  float bwd_start[8][SEGS];  // backward segment w's metrics at its end a1 after training
+  float fwd_end[8][SEGS];    // forward segment w's metrics at a1
   uint32_t crc_part[2 * SEGS / 32];  // per-warp CRC syndromes
 };
 
-// The global loads of one 8-step chunk [8c, 8c + 8): the parity L-values and either
-// the systematic L-values (constituent 0) or the interleaver entries (constituent 1).
-// Every array read here is padded to Tp = 8 * nblk entries, so the vector loads stay
-// inside the frame's scratch even for the chunk holding the tail steps.
+// The global loads of one 8-step chunk: the parity L-values and either the systematic
+// L-values (constituent 0) or the 8 interleaved positions (constituent 1, in q0).
 struct RawChunk {
   float4 p0, p1;  // parity
-  uint4 q0, q1;   // systematic (as bits) or interleaver entries
+  uint4 q0, q1;   // systematic (as bits) or interleaved positions
 };
 
-__device__ __forceinline__ void load_raw(int j, int c, const Frame& fr, const uint32_t* __restrict__ perm,
-                                         RawChunk& r) {
-  const int t0 = c * kBlk;
-  const float* Lp = j == 0 ? fr.Lp0 : fr.Lp1;
-  r.p0 = __ldg(reinterpret_cast<const float4*>(Lp + t0));
-  r.p1 = __ldg(reinterpret_cast<const float4*>(Lp + t0) + 1);
-  const uint4* q = j == 0 ? reinterpret_cast<const uint4*>(fr.Ls + t0) : reinterpret_cast<const uint4*>(perm + t0);
-  r.q0 = __ldg(q);
-  r.q1 = __ldg(q + 1);
+__device__ __forceinline__ void load_raw(int j, int slot, const Frame& fr, RawChunk& r) {
+  const float4* Lp = reinterpret_cast<const float4*>(j == 0 ? fr.Lp0 : fr.Lp1) + slot;
+  r.p0 = __ldg(Lp);
+  r.p1 = __ldg(Lp + fr.m.slots);
+  if (j == 0) {
+    const uint4* q = reinterpret_cast<const uint4*>(fr.Ls) + slot;
+    r.q0 = __ldg(q);
+    r.q1 = __ldg(q + fr.m.slots);
+  } else {
+    r.q0 = __ldg(fr.perm + slot);
+  }
+}
+
+// Entry i of the 8 16-bit positions of a chunk.
+__device__ __forceinline__ uint32_t pos_of(const uint4& q, int i) {
+  const uint32_t w = i < 2 ? q.x : i < 4 ? q.y : i < 6 ? q.z : q.w;
+  return (i & 1) ? w >> 16 : w & 0xffffu;
 }
 
 // A chunk's a-priori and parity L-values.
@@ -374,15 +408,15 @@ __device__ __forceinline__ void resolve(int j, int c, int K, const Frame& fr, co
   ch.lp[0] = r.p0.x; ch.lp[1] = r.p0.y; ch.lp[2] = r.p0.z; ch.lp[3] = r.p0.w;
   ch.lp[4] = r.p1.x; ch.lp[5] = r.p1.y; ch.lp[6] = r.p1.z; ch.lp[7] = r.p1.w;
   if (j == 0) {
-    const float4 y0 = reinterpret_cast<const float4*>(Y + t0)[0];
-    const float4 y1 = reinterpret_cast<const float4*>(Y + t0)[1];
-    ch.la[0] = __uint_as_float(r.q0.x) + y0.x; ch.la[1] = __uint_as_float(r.q0.y) + y0.y;
-    ch.la[2] = __uint_as_float(r.q0.z) + y0.z; ch.la[3] = __uint_as_float(r.q0.w) + y0.w;
-    ch.la[4] = __uint_as_float(r.q1.x) + y1.x; ch.la[5] = __uint_as_float(r.q1.y) + y1.y;
-    ch.la[6] = __uint_as_float(r.q1.z) + y1.z; ch.la[7] = __uint_as_float(r.q1.w) + y1.w;
+    const float ls[kBlk] = {__uint_as_float(r.q0.x), __uint_as_float(r.q0.y), __uint_as_float(r.q0.z),
+                            __uint_as_float(r.q0.w), __uint_as_float(r.q1.x), __uint_as_float(r.q1.y),
+                            __uint_as_float(r.q1.z), __uint_as_float(r.q1.w)};
+    const float* y = Y + c;
+#pragma unroll
+    for (int i = 0; i < kBlk; ++i) ch.la[i] = ls[i] + y[i * fr.m.nblk];
   } else {
-    ch.la[0] = X[r.q0.x]; ch.la[1] = X[r.q0.y]; ch.la[2] = X[r.q0.z]; ch.la[3] = X[r.q0.w];
-    ch.la[4] = X[r.q1.x]; ch.la[5] = X[r.q1.y]; ch.la[6] = X[r.q1.z]; ch.la[7] = X[r.q1.w];
+#pragma unroll
+    for (int i = 0; i < kBlk; ++i) ch.la[i] = X[pos_of(r.q0, i)];
   }
   if (t0 + kBlk > K) {
 #pragma unroll
@@ -393,20 +427,20 @@ __device__ __forceinline__ void resolve(int j, int c, int K, const Frame& fr, co
   }
 }
 
-__device__ __forceinline__ void store_ck(float* ck, const float v[8]) {
-  float4* q = reinterpret_cast<float4*>(ck);
+__device__ __forceinline__ void store_ck(float* ck, int slots, int slot, const float v[8]) {
+  float4* q = reinterpret_cast<float4*>(ck) + slot;
   q[0] = make_float4(v[0], v[1], v[2], v[3]);
-  q[1] = make_float4(v[4], v[5], v[6], v[7]);
+  q[slots] = make_float4(v[4], v[5], v[6], v[7]);
 }
 
-__device__ __forceinline__ void load_ck(const float* ck, float v[8]) {
-  const float4* q = reinterpret_cast<const float4*>(ck);
-  const float4 c0 = q[0], c1 = q[1];
+__device__ __forceinline__ void load_ck(const float* ck, int slots, int slot, float v[8]) {
+  const float4* q = reinterpret_cast<const float4*>(ck) + slot;
+  const float4 c0 = q[0], c1 = q[slots];
   v[0] = c0.x; v[1] = c0.y; v[2] = c0.z; v[3] = c0.w;
   v[4] = c1.x; v[5] = c1.y; v[6] = c1.z; v[7] = c1.w;
 }
 
-__device__ __forceinline__ bool close8(const float* x, const float* y, Tol t) {
+__device__ __forceinline__ bool close8(const float x[8], const float y[8], Tol t) {
   bool ok = true;
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
@@ -416,51 +450,56 @@ __device__ __forceinline__ bool close8(const float* x, const float* y, Tol t) {
   return ok;
 }
 
-// One segment walk of constituent j, forward (fwd != 0) or backward.  The start
-// metrics are read from vin (shared memory).  Training steps outside the segment
-// run first without checkpoints -- forward over [t_train, a0), backward over
-// [a1, t_train) -- then the metrics at the segment boundary are written to vstart,
-// the segment's own steps run, leaving checkpoints at every multiple of 8 inside
-// [a0, a1) (and at T for the last backward segment), and the final metrics go to
-// vend.  Metrics are normalised at the end of every chunk, so every checkpoint and
-// both boundary vectors have their largest state at 0.  The global loads of chunk
-// c + 1 are issued before chunk c runs.  A fix-up walk (`refine`) starts from a
-// corrected boundary over checkpoints an earlier walk of the same segment left; it
-// stops at the first checkpoint its metrics reproduce (close8): from there on the
-// earlier walk is the same recursion, so its checkpoints and end stand.  Kept out of
-// line so that Phase A and the fix-up rounds share one copy of the code.
+// One segment walk of constituent j, forward (fwd != 0) or backward, of segment w from the
+// metrics v.  Training chunks outside the segment run first without checkpoints -- forward
+// over the `lead` chunks before it, backward over those behind it, cut short at the frame's
+// ends -- then the segment's own chunks run, leaving a checkpoint before each (and at T for
+// the last backward segment).  The metrics at the segment's end go to vbound (forward), or
+// those at its boundary after training (backward), [8][segs].  Walkers with a full training
+// stand at the same chunk of their segments, those that start at the frame's end at the
+// same chunk of the frame, so a warp's loads stay contiguous or equal.  Metrics are
+// normalised at the end of every chunk, so every checkpoint and both boundary vectors
+// have their largest state at 0.  The global loads of the next chunk are issued before a
+// chunk runs.  A fix-up walk (`refine`) starts from a corrected boundary over checkpoints
+// an earlier walk of the same segment left; it stops at the first checkpoint its metrics
+// reproduce (close8): from there on the earlier walk is the same recursion, so its
+// checkpoints and end stand.  Kept out of line so that Phase A and the fix-up rounds share
+// one copy of the code.
 template <int ALG>
-__device__ __noinline__ void segment_walk(int fwd, int j, int t_train, int a0, int a1, const float* vin, float* vstart,
-                                          float* vend, int K, int T, Frame fr, const float* X, const float* Y,
-                                          const uint32_t* perm, bool refine, Tol tol) {
-  float v[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) v[s] = vin[s];
+__device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float4 va, float4 vb, float* vbound, int segs,
+                                          int K, int T, Frame fr, const float* X, const float* Y, bool refine, Tol tol) {
+  float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+  const int Lc = fr.m.Lc, Sp = fr.m.Sp, slots = fr.m.slots, nblk = fr.m.nblk;
+  const int turn = (Lc - 1) * Sp - 1;  // from a segment's last slot back to the next one's first
+  const int c_own = w * Lc;
   if (fwd) {
-    const int c_end = (a1 + kBlk - 1) / kBlk;
-    int c = t_train / kBlk;
+    const int c_end = min(nblk, c_own + Lc);
+    int c = max(0, c_own - lead), kk = c % Lc;
+    int slot = kk * Sp + c / Lc;
     RawChunk nxt;
-    load_raw(j, c, fr, perm, nxt);
+    load_raw(j, slot, fr, nxt);
     for (; c < c_end; ++c) {
       const RawChunk cur = nxt;
-      if (c + 1 < c_end) load_raw(j, c + 1, fr, perm, nxt);
-      const int t0 = c * kBlk;
-      if (t0 == a0 && vstart) {
-#pragma unroll
-        for (int s = 0; s < 8; ++s) vstart[s] = v[s];
+      const int here = slot;
+      if (++kk == Lc) {
+        kk = 0;
+        slot -= turn;
+      } else {
+        slot += Sp;
       }
-      if (t0 >= a0) {
-        if (refine && t0 > a0) {
+      if (c + 1 < c_end) load_raw(j, slot, fr, nxt);
+      if (c >= c_own) {
+        if (refine && c > c_own) {
           float old[8];
-          load_ck(fr.cka + c * 8, old);
+          load_ck(fr.cka, slots, here, old);
           if (close8(v, old, tol)) return;
         }
-        store_ck(fr.cka + c * 8, v);
+        store_ck(fr.cka, slots, here, v);
       }
       Chunk ch;
       resolve(j, c, K, fr, X, Y, cur, ch);
-      const int n = min(kBlk, a1 - t0);
-      if (n == kBlk) {  // every chunk but the frame's last: no per-step tests
+      const int n = min(kBlk, T - c * kBlk);
+      if (n == kBlk) {  // every chunk but the frame's last, whose few steps run in a loop
 #pragma unroll
         for (int i = 0; i < kBlk; ++i) {
           Gam g;
@@ -468,37 +507,46 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int t_train, int a0, i
           fwd_step<ALG>(v, g);
         }
       } else {
+#pragma unroll 1
+        for (int i = 0; i < n; ++i) {
+          Gam g;
+          g.set(ch.la[0], ch.lp[0]);
+          fwd_step<ALG>(v, g);
 #pragma unroll
-        for (int i = 0; i < kBlk; ++i) {
-          if (i < n) {
-            Gam g;
-            g.set(ch.la[i], ch.lp[i]);
-            fwd_step<ALG>(v, g);
+          for (int q = 0; q + 1 < kBlk; ++q) {
+            ch.la[q] = ch.la[q + 1];
+            ch.lp[q] = ch.lp[q + 1];
           }
         }
       }
       normalize8(v);
     }
-  } else {
-    const int nblk = (T + kBlk - 1) / kBlk;
-    if (t_train == a1) {
-      if (vstart) {
 #pragma unroll
-        for (int s = 0; s < 8; ++s) vstart[s] = v[s];
-      }
-      if (a1 == T) store_ck(fr.ckb + nblk * 8, v);
+    for (int s = 0; s < 8; ++s) vbound[s * segs + w] = v[s];
+  } else {
+    int c = min(nblk, c_own + Lc + lead) - 1, kk = c % Lc;
+    int slot = kk * Sp + c / Lc;
+    if (lead == 0 || w == fr.m.S - 1) {
+#pragma unroll
+      for (int s = 0; s < 8; ++s) vbound[s * segs + w] = v[s];
+      if (w == fr.m.S - 1) store_ck(fr.ckb, slots, fr.m.slot_of(nblk), v);
     }
-    const int c_lo = a0 / kBlk;
-    int c = (t_train - 1) / kBlk;
     RawChunk nxt;
-    load_raw(j, c, fr, perm, nxt);
-    for (; c >= c_lo; --c) {
+    load_raw(j, slot, fr, nxt);
+    for (; c >= c_own; --c) {
       const RawChunk cur = nxt;
-      if (c - 1 >= c_lo) load_raw(j, c - 1, fr, perm, nxt);
+      const int here = slot;
+      if (--kk < 0) {
+        kk = Lc - 1;
+        slot += turn;
+      } else {
+        slot -= Sp;
+      }
+      if (c > c_own) load_raw(j, slot, fr, nxt);
       Chunk ch;
       resolve(j, c, K, fr, X, Y, cur, ch);
-      const int hi = min(kBlk, t_train - c * kBlk);
-      if (hi == kBlk) {  // every chunk but the frame's last: no per-step tests
+      const int hi = min(kBlk, T - c * kBlk);
+      if (hi == kBlk) {  // as in the forward walk
 #pragma unroll
         for (int i = kBlk - 1; i >= 0; --i) {
           Gam g;
@@ -506,34 +554,35 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int t_train, int a0, i
           bwd_step<ALG>(v, g);
         }
       } else {
-#pragma unroll
+#pragma unroll 1
         for (int i = kBlk - 1; i >= 0; --i) {
           if (i < hi) {
             Gam g;
-            g.set(ch.la[i], ch.lp[i]);
+            g.set(ch.la[kBlk - 1], ch.lp[kBlk - 1]);
             bwd_step<ALG>(v, g);
+          }
+#pragma unroll
+          for (int q = kBlk - 1; q > 0; --q) {
+            ch.la[q] = ch.la[q - 1];
+            ch.lp[q] = ch.lp[q - 1];
           }
         }
       }
       normalize8(v);
-      const int tm = c * kBlk;  // v now holds the metrics at time tm
-      if (tm == a1 && vstart) {
+      // v now holds the metrics before chunk c
+      if (c == c_own + Lc) {
 #pragma unroll
-        for (int s = 0; s < 8; ++s) vstart[s] = v[s];
+        for (int s = 0; s < 8; ++s) vbound[s * segs + w] = v[s];
       }
-      if (tm >= a0 && tm < a1) {
+      if (c < c_own + Lc) {
         if (refine) {
           float old[8];
-          load_ck(fr.ckb + c * 8, old);
+          load_ck(fr.ckb, slots, here, old);
           if (close8(v, old, tol)) return;
         }
-        store_ck(fr.ckb + c * 8, v);
+        store_ck(fr.ckb, slots, here, v);
       }
     }
-  }
-  if (vend) {
-#pragma unroll
-    for (int s = 0; s < 8; ++s) vend[s] = v[s];
   }
 }
 
@@ -554,16 +603,18 @@ struct SoftSink {
 // soDecode's last iteration, which also records every step's extrinsic value (tail
 // steps too) and parity extrinsic value in `sink`.
 template <int ALG, bool FULL, bool SOFT>
-__device__ __forceinline__ void ext_block(int j, int b, int K, int T, const Frame& fr, const float* X, const float* Y,
-                                          const uint32_t* perm, float sf, float* out, const SoftSink& sink) {
+__device__ __forceinline__ void ext_block(int j, int k, int w, int K, int T, const Frame& fr, const float* X,
+                                          const float* Y, float sf, float* out, const SoftSink& sink) {
+  const int b = w * fr.m.Lc + k, slot = k * fr.m.Sp + w, slots = fr.m.slots;
+  const int after = k + 1 < fr.m.Lc ? slot + fr.m.Sp : w + 1;  // chunk b + 1
   const int t0 = b * kBlk;
   const int n = FULL ? kBlk : min(kBlk, T - t0);
   RawChunk raw;
-  load_raw(j, b, fr, perm, raw);
+  load_raw(j, slot, fr, raw);
   float al[kBlk][8];
-  load_ck(fr.cka + b * 8, al[0]);
+  load_ck(fr.cka, slots, slot, al[0]);
   float be[8];
-  load_ck(fr.ckb + (b + 1) * 8, be);
+  load_ck(fr.ckb, slots, after, be);
   Chunk in;
   resolve(j, b, K, fr, X, Y, raw, in);
 #pragma unroll
@@ -579,7 +630,6 @@ __device__ __forceinline__ void ext_block(int j, int b, int K, int T, const Fram
   const float ls[kBlk] = {__uint_as_float(raw.q0.x), __uint_as_float(raw.q0.y), __uint_as_float(raw.q0.z),
                           __uint_as_float(raw.q0.w), __uint_as_float(raw.q1.x), __uint_as_float(raw.q1.y),
                           __uint_as_float(raw.q1.z), __uint_as_float(raw.q1.w)};
-  const uint32_t pq[kBlk] = {raw.q0.x, raw.q0.y, raw.q0.z, raw.q0.w, raw.q1.x, raw.q1.y, raw.q1.z, raw.q1.w};
 #pragma unroll
   for (int i = kBlk - 1; i >= 0; --i) {
     if (FULL || i < n) {
@@ -587,10 +637,10 @@ __device__ __forceinline__ void ext_block(int j, int b, int K, int T, const Fram
       g.set(in.la[i], in.lp[i]);
       const float e = sf * ext_step<ALG>(al[i], be, g);
       if (FULL || t0 + i < K) {
-        if (j == 0) out[t0 + i] = ls[i] + e;
-        else out[pq[i]] = e;
+        if (j == 0) out[i * fr.m.nblk + b] = ls[i] + e;
+        else out[pos_of(raw.q0, i)] = e;
       }
-      if (SOFT) {
+      if (SOFT && sink.ext) {
         sink.ext[t0 + i] = e;
         if (sink.par) store_llr(sink.par, sink.dtype, sink.par0 + t0 + i, par_step<ALG>(al[i], be, g));
       }
@@ -599,13 +649,74 @@ __device__ __forceinline__ void ext_block(int j, int b, int K, int T, const Fram
   }
 }
 
+// The same block for the log-MAP algorithms, step by step: their steps are long (dozens of
+// instructions per log-sum), and 8 of them unrolled three times over ran from the
+// instruction cache's misses.  The forward vectors wait in local memory.
+template <int ALG, bool SOFT>
+__device__ __forceinline__ void ext_steps(int j, int k, int w, int K, int T, const Frame& fr, const float* X, const float* Y,
+                                          float sf, float* out, const SoftSink& sink) {
+  const int b = w * fr.m.Lc + k, slot = k * fr.m.Sp + w, slots = fr.m.slots;
+  const int after = k + 1 < fr.m.Lc ? slot + fr.m.Sp : w + 1;  // chunk b + 1
+  const int t0 = b * kBlk, n = min(kBlk, T - t0);
+  RawChunk raw;
+  load_raw(j, slot, fr, raw);
+  float v[8], be[8];
+  load_ck(fr.cka, slots, slot, v);
+  load_ck(fr.ckb, slots, after, be);
+  Chunk in;
+  resolve(j, b, K, fr, X, Y, raw, in);
+  float4 al[kBlk][2];
+#pragma unroll 1
+  for (int i = 0;; ++i) {
+    al[i][0] = make_float4(v[0], v[1], v[2], v[3]);
+    al[i][1] = make_float4(v[4], v[5], v[6], v[7]);
+    if (i + 1 >= n) break;
+    Gam g;
+    g.set(in.la[i], in.lp[i]);
+    fwd_step<ALG>(v, g);
+  }
+  const uint32_t q[kBlk] = {raw.q0.x, raw.q0.y, raw.q0.z, raw.q0.w, raw.q1.x, raw.q1.y, raw.q1.z, raw.q1.w};
+#pragma unroll 1
+  for (int i = n - 1; i >= 0; --i) {
+    const float4 a0 = al[i][0], a1 = al[i][1];
+    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    Gam g;
+    g.set(in.la[i], in.lp[i]);
+    const float e = sf * ext_step<ALG>(a, be, g);
+    if (t0 + i < K) {
+      if (j == 0) out[i * fr.m.nblk + b] = __uint_as_float(q[i]) + e;
+      else out[(i & 1) ? q[i >> 1] >> 16 : q[i >> 1] & 0xffffu] = e;
+    }
+    if (SOFT && sink.ext) {
+      sink.ext[t0 + i] = e;
+      if (sink.par) store_llr(sink.par, sink.dtype, sink.par0 + t0 + i, par_step<ALG>(a, be, g));
+    }
+    if (i > 0) bwd_step<ALG>(be, g);
+  }
+}
+
+// Segment w and chunk k of block i in the order phase B takes the first n blocks: by k, and
+// within a k by w, so that the lanes of a warp read neighbouring slots.
+__device__ __forceinline__ void block_at(int i, int n, const LteMap& m, int& k, int& w) {
+  const int rem = n - (m.S - 1) * m.Lc;  // blocks of the last segment; the others have Lc
+  if (i < rem * m.S) {
+    k = i / m.S;
+    w = i - k * m.S;
+  } else {
+    const int q = (i - rem * m.S) / (m.S - 1);
+    k = rem + q;
+    w = i - rem * m.S - q * (m.S - 1);
+  }
+}
+
 // One frame's geometry and buffers, as the decode loop below sees them.
 struct LteJob {
-  int32_t K = 0, Kp = 0, Tp = 0, seg_len = 0, train = 0, iterations = 0;
+  int32_t K = 0, Kp = 0, Tp = 0, train = 0, iterations = 0;
+  LteMap map;
   const float* sf = nullptr;            // [2][iterations]
-  const uint32_t* perm = nullptr;       // interleaver of constituent 1, padded by 16 entries
-  const float* scratch = nullptr;       // staged L-values: Ls [Kp] | Lp0 [Tp] | Lp1 [Tp] | tail [8]
-  float* ck = nullptr;                  // checkpoints [2][nblk + 1][8]
+  const float* scratch = nullptr;       // staged L-values: Ls | Lp0 | Lp1 [8 slots] each | tail [8]
+  const uint4* perm = nullptr;          // staged interleaved positions [slots]
+  float* ck = nullptr;                  // checkpoints [2][8 slots]
   uint8_t* hard = nullptr;              // [K]
   int32_t* iters = nullptr;             // nullable
   unsigned long long* stats = nullptr;  // nullable
@@ -632,45 +743,57 @@ __host__ __device__ inline int lte_seg_len(int T, int segs) {
 
 // Decodes one frame with the whole CTA; smem holds 2 * Kp floats + Shared<SEGS>.
 // SOFT: soDecode (TurboDecoderImpl::soDecodeBlock, TurboDecoderImpl.cpp:75-150).
-template <int ALG, int SEGS, bool SOFT = false>
+// WHOLE: K is a multiple of 8, as every LTE size is (the max-log kernels have a form for each,
+// so that none carries both: their code has to stay in the instruction cache).
+template <int ALG, int SEGS, bool SOFT, bool WHOLE>
 __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
   constexpr int kThreads = 2 * SEGS;
   const int K = q.K, T = q.K + 3;
-  const int nblk = (T + kBlk - 1) / kBlk;
+  const LteMap& m = q.map;
+  const int nblk = m.nblk;
   const int nblk_msg = (K + kBlk - 1) / kBlk;
   float* X = smem;
   float* Y = smem + q.Kp;
   Shared<SEGS>& sh = *reinterpret_cast<Shared<SEGS>*>(smem + 2 * q.Kp);
   Frame fr;
-  const float* base = q.scratch;
-  fr.Ls = base;
-  fr.Lp0 = base + q.Kp;
-  fr.Lp1 = base + q.Kp + q.Tp;
-  fr.ts = base + q.Kp + 2 * q.Tp;
+  fr.m = m;
+  fr.Ls = q.scratch;
+  fr.Lp0 = q.scratch + 8 * m.slots;
+  fr.Lp1 = q.scratch + 16 * m.slots;
+  fr.ts = q.scratch + 24 * m.slots;
+  fr.perm = q.perm;
   fr.cka = q.ck;
-  fr.ckb = fr.cka + (nblk + 1) * 8;
+  fr.ckb = q.ck + 8 * m.slots;
   const int tid = threadIdx.x;
-  const int L = q.seg_len;
-  const int S = (T + L - 1) / L;
+  const int Lc = m.Lc, S = m.S;
   const Tol tol = SOFT ? kSoftTol : kDecodeTol;
 
+  if (ALG == kLinear && tid < 8) s_lut[tid] = c_lut.v[tid];
   // X = Ls + e0 with e0 = 0 (constituent 1 reads it first under Parallel scheduling)
-  for (int k = tid; k < q.Kp; k += kThreads) {
-    X[k] = fr.Ls[k];
-    Y[k] = 0.0f;
+  for (int i = tid; i < nblk; i += kThreads) {
+    int k, w;
+    block_at(i, nblk, m, k, w);
+    float l[8];
+    load_ck(fr.Ls, m.slots, k * m.Sp + w, l);
+#pragma unroll
+    for (int u = 0; u < kBlk; ++u) {
+      X[u * nblk + w * Lc + k] = l[u];
+      Y[u * nblk + w * Lc + k] = 0.0f;
+    }
   }
-  if (tid < 8) {
-    sh.flat[tid] = 0.0f;
-    sh.term[tid] = tid == 0 ? 0.0f : kNegInf;  // Tail: the trellis starts and ends in state 0
-  }
+  // Tail: the trellis starts and ends in state 0; training starts from all states equal
+  const float4 flat = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float4 term_a = make_float4(0.0f, kNegInf, kNegInf, kNegInf);
+  const float4 term_b = make_float4(kNegInf, kNegInf, kNegInf, kNegInf);
   __syncthreads();
   if (SOFT && q.state_in) {
     // the initial extrinsic values: X = Ls + e0, Y[pi(t)] = e1(t) (tail values are
     // replaced by the channel's tail bits before every pass, as in the reference)
     const int64_t s0 = q.frame * int64_t(2 * (K + 3));
+    const uint16_t* perm = reinterpret_cast<const uint16_t*>(fr.perm);
     for (int k = tid; k < K; k += kThreads) {
-      X[k] = fr.Ls[k] + load_llr(q.state_in, q.in_dtype, s0 + k);
-      Y[__ldg(q.perm + k)] = load_llr(q.state_in, q.in_dtype, s0 + K + 3 + k);
+      X[m.pos(k)] = X[m.pos(k)] + load_llr(q.state_in, q.in_dtype, s0 + k);
+      Y[perm[m.slot_of(k >> 3) * 8 + (k & 7)]] = load_llr(q.state_in, q.in_dtype, s0 + K + 3 + k);
     }
     __syncthreads();
   }
@@ -680,29 +803,17 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
     const bool last_soft = SOFT && it == q.iterations - 1;
     for (int jj = 0; jj < 2; ++jj) {
       const int j = q.parallel ? 1 - jj : jj;  // parallel: constituent 1 first, on the old X
-      const uint32_t* perm = q.perm;
+      const bool fwd = tid < SEGS;
+      const int w = fwd ? tid : tid - SEGS;
+      const int lead = q.train / kBlk;
       // ---- A: segments with training starts
       {
-        const bool fwd = tid < SEGS;
-        const int w = fwd ? tid : tid - SEGS;
-        if (w < S) {
-          const int a0 = w * L, a1 = min(T, a0 + L);
-          int t_train;
-          const float* vin;
-          if (fwd) {
-            const bool exact = (w == 0 || a0 - q.train <= 0);
-            t_train = exact ? 0 : a0 - q.train;
-            vin = exact ? sh.term : sh.flat;
-          } else {
-            const bool exact = (w == S - 1 || a1 + q.train >= T);
-            t_train = exact ? T : a1 + q.train;
-            vin = exact ? sh.term : sh.flat;
-          }
-          // a forward start is the checkpoint at a0, a backward end the one at a0
-          segment_walk<ALG>(fwd, j, t_train, a0, a1, vin, fwd ? nullptr : sh.bwd_start[w], fwd ? sh.fwd_end[w] : nullptr,
-                            K, T, fr, X,
-                            Y, perm, false, tol);
-        }
+        // the trellis's own start (end) where the training would reach it
+        const bool exact = fwd ? (w == 0 || w * Lc - lead <= 0) : (w == S - 1 || ((w + 1) * Lc + lead) * kBlk >= T);
+        // a forward start is the checkpoint at a0, a backward end the one at a0
+        if (w < S)
+          segment_walk<ALG>(fwd, j, w, lead, exact ? term_a : flat, exact ? term_b : flat,
+                            fwd ? &sh.fwd_end[0][0] : &sh.bwd_start[0][0], SEGS, K, T, fr, X, Y, false, tol);
       }
       __syncthreads();
       // ---- A2: verify boundaries; walk again the segments whose start disagrees.
@@ -710,40 +821,34 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
       // boundary adds two more.
       int rounds = 0;
       for (int round = 0; round < S; ++round) {
-        const bool fwd = tid < SEGS;
-        const int w = fwd ? tid : tid - SEGS;
         bool bad = false;
-        if (w < S) {
-          // forward: this segment's start (its checkpoint at a0) against the previous
-          // segment's end; backward: this segment's start at a1 against the next
-          // segment's end (its checkpoint at a1)
-          if (fwd && w > 0) bad = !close8(fr.cka + (w * L / kBlk) * 8, sh.fwd_end[w - 1], tol);
-          if (!fwd && w < S - 1) bad = !close8(sh.bwd_start[w], fr.ckb + ((w + 1) * L / kBlk) * 8, tol);
+        // forward: this segment's start (its checkpoint at a0) against the previous
+        // segment's end; backward: this segment's start at a1 against the next
+        // segment's end (its checkpoint at a1).  `right` is the neighbour's end.
+        float right[8] = {};
+        if (w < S && (fwd ? w > 0 : w < S - 1)) {
+          float mine[8];
+          if (fwd) {
+            load_ck(fr.cka, m.slots, w, mine);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) right[s] = sh.fwd_end[s][w - 1];
+          } else {
+            load_ck(fr.ckb, m.slots, w + 1, right);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) mine[s] = sh.bwd_start[s][w];
+          }
+          bad = !close8(mine, right, tol);
         }
-        if (!__syncthreads_or(bad)) break;
-        ++rounds;
-        // Walk every rejected segment again from its neighbour's end.  The end is
-        // copied to registers before the barrier and becomes the segment's start
+        // The end is in registers before the barrier and becomes the segment's start
         // after it, so a neighbour that is itself being walked again is read in its
         // old state; the next round checks the boundary again.
-        float start[8];
-        if (bad) {
-#pragma unroll
-          for (int s = 0; s < 8; ++s) start[s] = fwd ? sh.fwd_end[w - 1][s] : fr.ckb[((w + 1) * L / kBlk) * 8 + s];
-        }
-        __syncthreads();
+        if (!__syncthreads_or(bad)) break;
+        ++rounds;
         if (bad) {
           if (q.stats) atomicAdd(q.stats + 2, 1ull);
-          // the walk reads its start from sv: a forward segment's checkpoint at a0
-          // (which the walk writes again with the same values), a backward segment's
-          // start vector
-          float* sv = fwd ? fr.cka + (w * L / kBlk) * 8 : sh.bwd_start[w];
-#pragma unroll
-          for (int s = 0; s < 8; ++s) sv[s] = start[s];
-          const int a0 = w * L, a1 = min(T, a0 + L);
-          segment_walk<ALG>(fwd, j, fwd ? a0 : a1, a0, a1, sv, fwd ? nullptr : sv, fwd ? sh.fwd_end[w] : nullptr, K, T, fr,
-                            X, Y, perm, true,
-                            tol);
+          segment_walk<ALG>(fwd, j, w, 0, make_float4(right[0], right[1], right[2], right[3]),
+                            make_float4(right[4], right[5], right[6], right[7]),
+                            fwd ? &sh.fwd_end[0][0] : &sh.bwd_start[0][0], SEGS, K, T, fr, X, Y, true, tol);
         }
         __syncthreads();
       }
@@ -758,31 +863,27 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
       // soDecode does not scale the extrinsic values (TurboDecoderImpl.cpp:75-150)
       const float sf = SOFT ? 1.0f : q.sf[j * q.iterations + it];
       float* out = j == 0 ? X : (q.parallel ? q.ynew : Y);
+      // soDecode's last iteration runs every block, tail blocks too, and records the
+      // extrinsic and parity extrinsic values
+      const int blocks = last_soft ? nblk : nblk_msg;
+      SoftSink sink;
       if (last_soft) {
-        // soDecode's last iteration: every block, tail blocks too, recording the
-        // extrinsic and parity extrinsic values
-        SoftSink sink;
         sink.ext = q.soft_ext + j * q.Tp;
         sink.par = q.parity_out;
         sink.par0 = q.frame * int64_t(3 * K + 12) + K + 6 + j * (K + 3);
         sink.dtype = q.out_dtype;
-        for (int b = tid; b < nblk; b += kThreads) ext_block<ALG, false, true>(j, b, K, T, fr, X, Y, perm, sf, out, sink);
-      } else {
-        const SoftSink none;
-        for (int b = tid; b < nblk_msg; b += kThreads) {
-          // in max-log a block of 8 message steps (every block but, when K is not a
-          // multiple of 8, the last) runs without per-step tests (the log-MAP kernels
-          // keep one form, which their registers hold without spilling)
-          if (ALG == kApproximate && b * kBlk + kBlk <= K)
-            ext_block<ALG, true, false>(j, b, K, T, fr, X, Y, perm, sf, out, none);
-          else
-            ext_block<ALG, false, false>(j, b, K, T, fr, X, Y, perm, sf, out, none);
-        }
+      }
+      for (int i = tid; i < blocks; i += kThreads) {
+        int kb, wb;
+        block_at(i, blocks, m, kb, wb);
+        // WHOLE: every message block has 8 message steps, and runs without per-step tests
+        if constexpr (ALG == kApproximate) ext_block<ALG, WHOLE && !SOFT, SOFT>(j, kb, wb, K, T, fr, X, Y, sf, out, sink);
+        else ext_steps<ALG, SOFT>(j, kb, wb, K, T, fr, X, Y, sf, out, sink);
       }
       __syncthreads();
     }
     if (q.parallel) {
-      for (int k = tid; k < K; k += kThreads) Y[k] = q.ynew[k];
+      for (int k = tid; k < K; k += kThreads) Y[m.pos(k)] = q.ynew[m.pos(k)];
       __syncthreads();
     }
     // CRC stop (an extension; LTE transport blocks end with a CRC-24): the decisions
@@ -791,7 +892,7 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
     if (q.crc) {
       uint32_t syn = 0;
       for (int k = tid; k < K; k += kThreads)
-        if ((X[k] + Y[k]) > 0.0f) syn ^= __ldg(q.crc + k);
+        if ((X[m.pos(k)] + Y[m.pos(k)]) > 0.0f) syn ^= __ldg(q.crc + k);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) syn ^= __shfl_xor_sync(0xffffffffu, syn, o);
       if ((tid & 31) == 0) sh.crc_part[tid >> 5] = syn;
@@ -816,11 +917,14 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
     const int64_t f = q.frame;
     for (int k = tid; k < K + 6; k += kThreads) {
       float v;
-      if (k < K) v = e0[k] + Y[k];
+      if (k < K) v = e0[k] + Y[m.pos(k)];
       else v = k < K + 3 ? e0[k] : e1[k - 3];
       if (q.syst_out) store_llr(q.syst_out, q.out_dtype, f * int64_t(K + 6) + k, v);
       if (q.parity_out) store_llr(q.parity_out, q.out_dtype, f * int64_t(3 * K + 12) + k, v);
-      if (q.msg_out && k < K) store_llr(q.msg_out, q.out_dtype, f * int64_t(K) + k, fr.Ls[k] + v);
+      if (q.msg_out && k < K) {
+        const float ls = fr.Ls[((k >> 2) & 1) * 4 * m.slots + m.slot_of(k >> 3) * 4 + (k & 3)];
+        store_llr(q.msg_out, q.out_dtype, f * int64_t(K) + k, ls + v);
+      }
     }
     if (q.state_out)
       for (int t = tid; t < 2 * (K + 3); t += kThreads) {
@@ -829,34 +933,45 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
       }
   } else {
     // a-posteriori and hard decision, TurboDecoderImpl.cpp:64-71
-    for (int k = tid; k < K; k += kThreads) q.hard[k] = uint8_t((X[k] + Y[k]) > 0.0f);
+    if (K % 8 == 0 && reinterpret_cast<uintptr_t>(q.hard) % 8 == 0) {
+      for (int b = tid; b < K / 8; b += kThreads) {
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          lo |= uint32_t((X[i * nblk + b] + Y[i * nblk + b]) > 0.0f) << (8 * i);
+          hi |= uint32_t((X[(i + 4) * nblk + b] + Y[(i + 4) * nblk + b]) > 0.0f) << (8 * i);
+        }
+        reinterpret_cast<uint2*>(q.hard)[b] = make_uint2(lo, hi);
+      }
+    } else {
+      for (int k = tid; k < K; k += kThreads) q.hard[k] = uint8_t((X[m.pos(k)] + Y[m.pos(k)]) > 0.0f);
+    }
     if (q.iters && tid == 0) *q.iters = ran;
   }
 }
 
-template <int ALG, int SEGS, bool SOFT = false>
+template <int ALG, int SEGS, bool SOFT, bool WHOLE>
 __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : (SEGS == 128 ? 1 : 3)) turbo_lte_kernel(TurboLteParams p) {
   extern __shared__ float smem[];
   const int64_t f = p.frame0 + blockIdx.x;
-  const int nblk = (p.K + 3 + kBlk - 1) / kBlk;
   LteJob q;
   q.K = p.K;
   q.Kp = p.Kp;
   q.Tp = p.Tp;
-  q.seg_len = p.seg_len;
+  q.map = LteMap{p.seg_len / kBlk, p.segments, p.seg_stride, p.slots, p.Tp / kBlk};
   q.train = p.train;
   q.iterations = p.iterations;
   q.sf = p.sf;
-  q.perm = p.perm[1];
-  q.scratch = p.scratch + f * p.frame_stride;
-  q.ck = p.ck + f * int64_t(2 * (nblk + 1) * 8);
+  q.perm = p.perm_pos;
+  q.scratch = p.scratch + int64_t(blockIdx.x) * p.frame_stride;
+  q.ck = p.ck + int64_t(blockIdx.x) * (16 * p.slots);
   q.hard = p.hard + f * p.K;
   q.iters = p.iters ? p.iters + f : nullptr;
   q.stats = p.stats;
   q.crc = p.crc;
   q.parallel = p.parallel;
   if (p.ynew) {  // per frame: ynew [Tp] | soft_ext [2][Tp]
-    q.ynew = p.ynew + f * int64_t(3 * p.Tp);
+    q.ynew = p.ynew + int64_t(blockIdx.x) * (3 * p.Tp);
     q.soft_ext = q.ynew + p.Tp;
   }
   q.state_in = p.state_in;
@@ -867,7 +982,7 @@ __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : (SEGS == 128 ? 1 : 
   q.parity_out = p.parity_out;
   q.state_out = p.state_out;
   q.frame = f;
-  decode_lte_frame<ALG, SEGS, SOFT>(q, smem);
+  decode_lte_frame<ALG, SEGS, SOFT, WHOLE>(q, smem);
 }
 
 
@@ -876,85 +991,108 @@ __device__ __forceinline__ float to_f32(T v) { return float(v); }
 template <>
 __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
 
-// Input [f][3K+12] in FeCl's turbo layout -> padded FP32 scratch, one block per frame
-// (grid-strided over frames): the systematic, parity and tail regions are copied by
-// loops of their own, so no element needs a division to find its place, and the
-// element type is fixed per launch.
-template <typename T>
-__global__ void turbo_lte_stage(TurboLteParams p) {
-  const T* llr = static_cast<const T*>(p.llr);
-  const int K = p.K, Kp = p.Kp, Tp = p.Tp;
-  for (int64_t f = blockIdx.x; f < p.nframes; f += gridDim.x) {
-    const T* in = llr + f * int64_t(3 * K + 12);
-    float* out = p.scratch + f * p.frame_stride;
-    // soDecode's a-priori input is added to the channel's systematic values and tails
-    // (TurboDecoderImpl.cpp:77-82)
-    const T* sys = p.syst_in ? static_cast<const T*>(p.syst_in) + f * int64_t(K + 6) : nullptr;
-    // four elements per thread and step, all loaded before any is stored, so that each
-    // thread keeps four loads in flight (load latency, not bandwidth, bounds the copy)
-    constexpr int kU = 4;
-    const int step = int(blockDim.x);
-    for (int i0 = threadIdx.x; i0 < Kp; i0 += kU * step) {
-      float v[kU];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int i = i0 + u * step;
-        v[u] = i < K ? (sys ? to_f32(in[i]) + to_f32(sys[i]) : to_f32(in[i])) : 0.0f;
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u)
-        if (i0 + u * step < Kp) out[i0 + u * step] = v[u];
-    }
-    for (int c = 0; c < 2; ++c) {
-      const T* src = in + K + 6 + c * (K + 3);  // parity (with its tail) of constituent c
-      float* dst = out + Kp + c * Tp;
-      for (int t0 = threadIdx.x; t0 < Tp; t0 += kU * step) {
-        float v[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          const int t = t0 + u * step;
-          v[u] = t < K + 3 ? to_f32(src[t]) : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u)
-          if (t0 + u * step < Tp) dst[t0 + u * step] = v[u];
-      }
-    }
-    if (threadIdx.x < 8) {
-      float v = 0.0f;
-      if (threadIdx.x < 6) v = sys ? to_f32(in[K + threadIdx.x]) + to_f32(sys[K + threadIdx.x]) : to_f32(in[K + threadIdx.x]);
-      out[Kp + 2 * Tp + threadIdx.x] = v;
-    }
-  }
-}
-
-// Geometry of a frame of K message bits: T trellis steps, nblk 8-step blocks, the
-// padded systematic / parity lengths Kp = Tp, the staged-input stride and the
-// segment length of the `segs` forward and `segs` backward segments.
+// Geometry of a frame of K message bits: T trellis steps, nblk 8-step chunks, the padded
+// length Kp = Tp of the exchange arrays, and the staged layout of `segs` forward and `segs`
+// backward segments (LteMap).  Sp is one more than S (the checkpoint at T may open a segment
+// of its own) and even, so that rows of slots start on 32-byte sectors.
 struct LteGeometry {
-  int T, nblk, Tp, Kp, stride, seg_len;
+  int T, nblk, Tp, Kp, seg_len, S, Sp, slots;
   __host__ __device__ LteGeometry(int K, int segs) {
     T = K + 3;
     nblk = (T + kBlk - 1) / kBlk;
     Tp = nblk * kBlk;
     Kp = Tp;
-    stride = Kp + 2 * Tp + 8;
     seg_len = lte_seg_len(T, segs);
+    S = (T + seg_len - 1) / seg_len;
+    Sp = (S + 2) & ~1;
+    slots = seg_len / kBlk * Sp;
   }
-  // Staged inputs then checkpoints, rounded to 128 bytes so frames share no cache line.
-  __host__ __device__ int frame_floats() const { return (stride + 2 * (nblk + 1) * 8 + 31) & ~31; }
+  __host__ __device__ LteMap map() const { return LteMap{seg_len / kBlk, S, Sp, slots, nblk}; }
+  __host__ __device__ int staged_floats() const { return 24 * slots + 8; }
+  __host__ __device__ int ck_floats() const { return 16 * slots; }
+  __host__ __device__ int perm_floats() const { return 4 * slots; }
+  // One frame of the mixed-K batch: staged inputs, checkpoints, positions, rounded to 128
+  // bytes so frames share no cache line.
+  __host__ __device__ int frame_floats() const { return (staged_floats() + ck_floats() + perm_floats() + 31) & ~31; }
 };
 
-// Stages element i of a frame's staged inputs from FeCl's turbo layout
-// | msg [K] | systTail1 [3] | systTail2 [3] | parity1 [K+3] | parity2 [K+3] |.
-__device__ __forceinline__ float staged_value(const void* llr, int dtype, int64_t in0, int K, int Kp, int Tp, int i) {
-  if (i < Kp) return i < K ? load_llr(llr, dtype, in0 + i) : 0.0f;
-  if (i < Kp + 2 * Tp) {
-    const int c = (i - Kp) / Tp, t = (i - Kp) % Tp;
-    return t < K + 3 ? load_llr(llr, dtype, in0 + K + 6 + c * (K + 3) + t) : 0.0f;
+// Quotients by Lc of chunk numbers (below 2^11) as a multiplication.
+__device__ __forceinline__ int staged_at(int t, const LteMap& m, uint32_t inv) {
+  const int c = t >> 3, w = int(__umulhi(uint32_t(c), inv)), slot = (c - w * m.Lc) * m.Sp + w;
+  return ((t >> 2) & 1) * 4 * m.slots + slot * 4 + (t & 3);
+}
+__device__ __forceinline__ uint32_t inverse_of(int d) { return d > 1 ? 0xffffffffu / uint32_t(d) + 1u : 0u; }
+
+// One frame's input [3K+12] in FeCl's turbo layout | msg [K] | systTail1 [3] | systTail2 [3] |
+// parity1 [K+3] | parity2 [K+3] | -> FP32 scratch in slot order: the regions are copied by
+// loops of their own, and the element type is fixed per launch.  soDecode's a-priori input is added
+// to the channel's systematic values and tails (TurboDecoderImpl.cpp:77-82).  Lc = 1 has
+// no quotient: chunk c is segment c.
+template <typename T>
+__device__ __forceinline__ void stage_frame(const T* in, const T* sys, float* out, int K, int Tp, const LteMap& m) {
+  const uint32_t inv = inverse_of(m.Lc);
+  auto at = [&](int t) {
+    if (m.Lc == 1) return ((t >> 2) & 1) * 4 * m.slots + (t >> 3) * 4 + (t & 3);
+    return staged_at(t, m, inv);
+  };
+  // four elements per thread and step, all loaded before any is stored, so that each
+  // thread keeps four loads in flight (load latency, not bandwidth, bounds the copy)
+  constexpr int kU = 4;
+  const int step = int(blockDim.x);
+  for (int i0 = threadIdx.x; i0 < Tp; i0 += kU * step) {
+    float v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int i = i0 + u * step;
+      v[u] = i < K ? (sys ? to_f32(in[i]) + to_f32(sys[i]) : to_f32(in[i])) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (i0 + u * step < Tp) out[at(i0 + u * step)] = v[u];
   }
-  const int t = i - Kp - 2 * Tp;
-  return t < 6 ? load_llr(llr, dtype, in0 + K + t) : 0.0f;
+  for (int c = 0; c < 2; ++c) {
+    const T* src = in + K + 6 + c * (K + 3);  // parity (with its tail) of constituent c
+    float* dst = out + (1 + c) * 8 * m.slots;
+    for (int t0 = threadIdx.x; t0 < Tp; t0 += kU * step) {
+      float v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int t = t0 + u * step;
+        v[u] = t < K + 3 ? to_f32(src[t]) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (t0 + u * step < Tp) dst[at(t0 + u * step)] = v[u];
+    }
+  }
+  if (threadIdx.x < 8) {
+    float v = 0.0f;
+    if (threadIdx.x < 6) v = sys ? to_f32(in[K + threadIdx.x]) + to_f32(sys[K + threadIdx.x]) : to_f32(in[K + threadIdx.x]);
+    out[24 * m.slots + threadIdx.x] = v;
+  }
+}
+
+// The interleaved position (LteMap::pos) of every step, 16 bits each, in slot order; steps
+// past K read position 0.
+__device__ __forceinline__ void stage_positions(const uint32_t* perm, uint16_t* out, int K, int Tp, const LteMap& m,
+                                                int first, int step) {
+  for (int t = first; t < Tp; t += step) out[m.slot_of(t >> 3) * 8 + (t & 7)] = t < K ? uint16_t(m.pos(int(perm[t]))) : 0;
+}
+
+// Staging of a launch's frames (grid-strided) and, by the last block, of its positions.
+template <typename T>
+__global__ void turbo_lte_stage(TurboLteParams p) {
+  const LteMap m{p.seg_len / kBlk, p.segments, p.seg_stride, p.slots, p.Tp / kBlk};
+  if (blockIdx.x == gridDim.x - 1) {
+    stage_positions(p.perm[1], reinterpret_cast<uint16_t*>(p.perm_pos), p.K, p.Tp, m, threadIdx.x, blockDim.x);
+    return;
+  }
+  const T* llr = static_cast<const T*>(p.llr);
+  for (int64_t i = blockIdx.x; i < p.nframes; i += gridDim.x - 1) {
+    const int64_t f = p.frame0 + i;
+    const T* sys = p.syst_in ? static_cast<const T*>(p.syst_in) + f * int64_t(p.K + 6) : nullptr;
+    stage_frame(llr + f * int64_t(3 * p.K + 12), sys, p.scratch + i * p.frame_stride, p.K, p.Tp, m);
+  }
 }
 
 // Mixed-K batch, staging: one block per frame (grid-strided).
@@ -962,15 +1100,21 @@ __global__ void turbo_lte_batch_stage(TurboLteBatchParams p) {
   for (int64_t f = blockIdx.x; f < p.nframes; f += gridDim.x) {
     const TurboLteBatchFrame d = p.frames[f];
     const LteGeometry g(d.K, kDefaultSegs);
-    for (int i = threadIdx.x; i < g.stride; i += blockDim.x)
-      d.scratch[i] = staged_value(d.llr, d.llr_dtype, 0, d.K, g.Kp, g.Tp, i);
+    const LteMap m = g.map();
+    switch (d.llr_dtype) {
+      case kF64: stage_frame(static_cast<const double*>(d.llr), static_cast<const double*>(nullptr), d.scratch, d.K, g.Tp, m); break;
+      case kF16: stage_frame(static_cast<const __half*>(d.llr), static_cast<const __half*>(nullptr), d.scratch, d.K, g.Tp, m); break;
+      default: stage_frame(static_cast<const float*>(d.llr), static_cast<const float*>(nullptr), d.scratch, d.K, g.Tp, m); break;
+    }
+    stage_positions(d.perm, reinterpret_cast<uint16_t*>(d.scratch + g.staged_floats() + g.ck_floats()), d.K, g.Tp, m,
+                    threadIdx.x, blockDim.x);
   }
 }
 
 // Mixed-K batch, decoding: persistent CTAs take frames from a counter in the order
 // of the descriptor table (longest first), so frames of every size share one launch
 // and the long ones do not trail behind.  Shared memory is sized for the largest K.
-template <int ALG, int SEGS>
+template <int ALG, int SEGS, bool WHOLE>
 __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : 3) turbo_lte_batch_kernel(TurboLteBatchParams p) {
   extern __shared__ float smem[];
   __shared__ int next;
@@ -986,18 +1130,18 @@ __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : 3) turbo_lte_batch_
     q.K = d.K;
     q.Kp = g.Kp;
     q.Tp = g.Tp;
-    q.seg_len = g.seg_len;
+    q.map = g.map();
     q.train = p.train;
     q.iterations = d.iterations;
     q.sf = d.sf;
-    q.perm = d.perm;
     q.scratch = d.scratch;
-    q.ck = d.scratch + g.stride;
+    q.ck = d.scratch + g.staged_floats();
+    q.perm = reinterpret_cast<const uint4*>(d.scratch + g.staged_floats() + g.ck_floats());
     q.hard = d.hard;
     q.iters = d.iters;
     q.stats = p.stats;
     q.crc = d.crc;
-    decode_lte_frame<ALG, SEGS>(q, smem);
+    decode_lte_frame<ALG, SEGS, false, WHOLE>(q, smem);
   }
 }
 
@@ -1025,17 +1169,10 @@ int device_sms() {
 // cost more than the training they save (Exact 54.8 ms with 80 against 40.7 ms).
 int default_train(int algorithm) { return algorithm == kApproximate ? 80 : 96; }
 
-// Resident CTAs of kern on the whole GPU (0 if the query fails).
-template <class Kern>
-int64_t resident_ctas(Kern kern, int threads, size_t smem) {
-  int per_sm = 0, dev = 0, sms = 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess ||
-      cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return int64_t(per_sm) * sms;
+// CTAs of `smem` bytes resident on an SM, at most `most` (their registers).
+int64_t ctas_per_sm(size_t smem, int64_t most) {
+  const int64_t fit = int64_t((228 << 10) / ((smem + 1024 + 127) / 128 * 128));
+  return fit < most ? fit : most;
 }
 
 // Frames (from the first) that the 32-segment shape decodes when the segment count
@@ -1045,31 +1182,11 @@ int64_t resident_ctas(Kern kern, int threads, size_t smem) {
 // frame's decode.  When the 64-segment shape (fewer resident CTAs: 3 per SM against
 // 4, register-bound) would end on a round less than half full, whole rounds of the
 // 32-segment shape go first so that the 64-segment rounds are full or nearly so:
-// K=6144 x 1024 frames on 148 SMs is 592 + 432 frames in two rounds (1.12 ms measured)
-// instead of 444 + 444 + 136 in three (1.23 ms).  Which frames take which shape does not
-// change their results beyond FP32 rounding of the window boundaries.
-template <int ALG>
-int64_t split_frames(int K, int64_t nframes) {
-  // resident CTAs of both shapes, remembered per (device, K)
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, std::pair<int64_t, int64_t>> known;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  int64_t r64, r32;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = known.find({dev, K});
-    if (it == known.end()) {
-      const std::pair<int64_t, int64_t> r{resident_ctas(turbo_lte_kernel<ALG, 64>, 128, lte_smem_bytes<64>(K)),
-                                          resident_ctas(turbo_lte_kernel<ALG, 32>, 64, lte_smem_bytes<32>(K))};
-      it = known.emplace(std::make_pair(dev, K), r).first;
-    }
-    r64 = it->second.first;
-    r32 = it->second.second;
-  }
+// K=6144 x 1024 frames on 148 SMs is 592 + 432 frames in two rounds instead of
+// 444 + 444 + 136 in three.  Which frames take which shape decides the FP32 rounding of
+// their window boundaries, so the rule is fixed arithmetic.
+int64_t split_frames(int K, int64_t nframes, int sms) {
+  const int64_t r64 = sms * ctas_per_sm(lte_smem_bytes<64>(K), 3), r32 = sms * ctas_per_sm(lte_smem_bytes<32>(K), 4);
   if (r64 <= 0 || r32 <= 0 || nframes <= r64) return 0;
   auto rounds = [](int64_t n, int64_t r) { return (n + r - 1) / r; };
   auto tail_ok = [&](int64_t n) { return n % r64 == 0 || 2 * (n % r64) >= r64; };
@@ -1087,130 +1204,118 @@ cudaError_t turbo_lte_init() {
   static std::atomic<unsigned long long> done{0};
   return once_per_device(done, [] {
     const LinearLut l = make_linear_lut();
-    return cudaMemcpyToSymbol(c_lut, &l, sizeof(l));
+    LinearPairs t;
+    for (int i = 0; i < 8; ++i) t.v[i] = i < 7 ? make_float2(l.y[i + 1] - l.y[i], l.y[i]) : make_float2(0.0f, 0.0f);
+    return cudaMemcpyToSymbol(c_lut, &t, sizeof(t));
   });
 }
 
 size_t turbo_lte_scratch_bytes(int K, int64_t nframes, bool extra) {
-  const int T = K + 3;
-  const int nblk = (T + kBlk - 1) / kBlk;
-  const int Tp = nblk * kBlk;
-  const int Kp = Tp;
-  const int64_t stride = Kp + 2 * Tp + 8;
-  return size_t(nframes) * (size_t(stride) + size_t(2 * (nblk + 1) * 8) + (extra ? size_t(3 * Tp) : 0)) * sizeof(float);
+  // whichever shapes the launcher takes: the largest frame of the three, and positions for two launches
+  int frame = 0, positions = 0;
+  for (int segs : {32, 64, 128}) {
+    const LteGeometry g(K, segs);
+    frame = std::max(frame, g.staged_floats() + g.ck_floats());
+    positions = std::max(positions, g.perm_floats());
+  }
+  const int Tp = LteGeometry(K, kDefaultSegs).Tp;
+  return (size_t(nframes) * (size_t(frame) + (extra ? size_t(3 * Tp) : 0)) + 2 * size_t(positions)) * sizeof(float);
 }
 
 cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
   cudaError_t e0 = turbo_lte_init();
   if (e0 != cudaSuccess) return e0;
   if (p.nframes <= 0) return cudaSuccess;
-  const int segs = resolve_segs(p.segs);
-  const LteGeometry g(p.K, segs);
-  p.Tp = g.Tp;
-  p.Kp = g.Kp;  // the systematic region and the exchange arrays are padded like the parity
-  p.frame_stride = g.stride;
-  p.ck = p.scratch + p.nframes * p.frame_stride;
-  // parallel scheduling and soDecode: per frame ynew [Tp] | soft_ext [2][Tp] after the
-  // checkpoints (turbo_lte_scratch_bytes(K, n, true))
-  p.ynew = (p.parallel || p.soft) ? p.ck + p.nframes * int64_t(2 * (g.nblk + 1) * 8) : nullptr;
-  if (p.soft) p.crc = nullptr;
-  p.seg_len = g.seg_len;
-  if (p.train < 0) p.train = default_train(p.algorithm);
-  const unsigned stage_blocks = unsigned(p.nframes < 148 * 8 ? p.nframes : 148 * 8);
-  switch (p.llr_dtype) {
-    case kF64: turbo_lte_stage<double><<<stage_blocks, 256, 0, s>>>(p); break;
-    case kF16: turbo_lte_stage<__half><<<stage_blocks, 256, 0, s>>>(p); break;
-    default: turbo_lte_stage<float><<<stage_blocks, 256, 0, s>>>(p); break;
-  }
-  auto launch = [&](auto kern, int threads, size_t smem) -> cudaError_t {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (err != cudaSuccess) return err;
-    kern<<<unsigned(p.nframes), threads, smem, s>>>(p);
-    return cudaGetLastError();
-  };
-  if (p.soft) {
-    const size_t smem = lte_smem_bytes<64>(p.K);
-    switch (p.algorithm) {
-      case kExact: return launch(turbo_lte_kernel<kExact, 64, true>, 128, smem);
-      case kLinear: return launch(turbo_lte_kernel<kLinear, 64, true>, 128, smem);
-      default: return launch(turbo_lte_kernel<kApproximate, 64, true>, 128, smem);
-    }
-  }
-  if (segs == 32) {
-    const size_t smem = lte_smem_bytes<32>(p.K);
-    switch (p.algorithm) {
-      case kExact: return launch(turbo_lte_kernel<kExact, 32>, 64, smem);
-      case kLinear: return launch(turbo_lte_kernel<kLinear, 32>, 64, smem);
-      default: return launch(turbo_lte_kernel<kApproximate, 32>, 64, smem);
-    }
-  }
+  int segs = resolve_segs(p.segs);
   // A batch of at most one frame per SM decodes in one round whose time is one
   // frame's latency: with the segment count left to the launcher it takes the
   // 128-segment shape (one CTA of 256 threads per frame: half as many phase B blocks
   // per thread and shorter segment walks than with 64), as does an explicit 128.
-  if (segs == 128 || (p.segs == 0 && p.nframes <= device_sms())) {
-    p.seg_len = LteGeometry(p.K, 128).seg_len;
-    const size_t smem = lte_smem_bytes<128>(p.K);
-    switch (p.algorithm) {
-      case kExact: return launch(turbo_lte_kernel<kExact, 128>, 256, smem);
-      case kLinear: return launch(turbo_lte_kernel<kLinear, 128>, 256, smem);
-      default: return launch(turbo_lte_kernel<kApproximate, 128>, 256, smem);
+  // soDecode always uses 64.
+  const int sms = device_sms();
+  if (p.soft) segs = 64;
+  else if (p.segs == 0 && p.nframes <= sms) segs = 128;
+  if (p.soft) p.crc = nullptr;
+  if (p.train < 0) p.train = default_train(p.algorithm);
+  float* at = p.scratch;
+  // frames [first, first + n) with `segs` segments: staging, then the decoder
+  auto decode = [&](int64_t first, int64_t n, int segs, auto kern, size_t smem) -> cudaError_t {
+    const LteGeometry g(p.K, segs);
+    TurboLteParams q = p;
+    q.frame0 = first;
+    q.nframes = n;
+    q.Tp = g.Tp;
+    q.Kp = g.Kp;  // the exchange arrays are padded like the parity
+    q.seg_len = g.seg_len;
+    q.segments = g.S;
+    q.seg_stride = g.Sp;
+    q.slots = g.slots;
+    q.frame_stride = g.staged_floats();
+    q.scratch = at;
+    q.ck = q.scratch + n * q.frame_stride;
+    at = q.ck + n * int64_t(g.ck_floats());
+    // parallel scheduling and soDecode: per frame ynew [Tp] | soft_ext [2][Tp] after the
+    // checkpoints (turbo_lte_scratch_bytes(K, n, true))
+    q.ynew = (p.parallel || p.soft) ? at : nullptr;
+    if (q.ynew) at += n * int64_t(3 * g.Tp);
+    q.perm_pos = reinterpret_cast<uint4*>(at);
+    at += g.perm_floats();
+    const unsigned blocks = unsigned(n < 148 * 8 ? n : 148 * 8) + 1;
+    switch (p.llr_dtype) {
+      case kF64: turbo_lte_stage<double><<<blocks, 256, 0, s>>>(q); break;
+      case kF16: turbo_lte_stage<__half><<<blocks, 256, 0, s>>>(q); break;
+      default: turbo_lte_stage<float><<<blocks, 256, 0, s>>>(q); break;
     }
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (err != cudaSuccess) return err;
+    kern<<<unsigned(n), 2 * segs, smem, s>>>(q);
+    return cudaGetLastError();
+  };
+  // the kernel of a shape for the algorithm and, in max-log, for K % 8
+  const bool whole = p.K % kBlk == 0;
+  auto pick = [&](auto shape, auto soft) -> void (*)(TurboLteParams) {
+    constexpr int kSegs = decltype(shape)::value;
+    constexpr bool kSoft = decltype(soft)::value;
+    if (p.algorithm == kExact) return turbo_lte_kernel<kExact, kSegs, kSoft, true>;
+    if (p.algorithm == kLinear) return turbo_lte_kernel<kLinear, kSegs, kSoft, true>;
+    if (kSoft || whole) return turbo_lte_kernel<kApproximate, kSegs, kSoft, true>;
+    return turbo_lte_kernel<kApproximate, kSegs, kSoft, kSoft>;
+  };
+  using S32 = std::integral_constant<int, 32>;
+  using S64 = std::integral_constant<int, 64>;
+  using S128 = std::integral_constant<int, 128>;
+  if (p.soft) return decode(0, p.nframes, 64, pick(S64{}, std::true_type{}), lte_smem_bytes<64>(p.K));
+  if (segs == 32) return decode(0, p.nframes, 32, pick(S32{}, std::false_type{}), lte_smem_bytes<32>(p.K));
+  if (segs == 128) return decode(0, p.nframes, 128, pick(S128{}, std::false_type{}), lte_smem_bytes<128>(p.K));
+  // the launcher's choice: whole rounds of the 32-segment shape first where that fills
+  // the rounds better (split_frames)
+  const int64_t n32 = p.segs == 0 ? split_frames(p.K, p.nframes, sms) : 0;
+  if (n32 > 0) {
+    const cudaError_t err = decode(0, n32, 32, pick(S32{}, std::false_type{}), lte_smem_bytes<32>(p.K));
+    if (err != cudaSuccess) return err;
   }
-  const size_t smem = lte_smem_bytes<64>(p.K);
-  if (p.segs == 0) {
-    // the launcher's choice: whole rounds of the 32-segment shape first where that
-    // fills the rounds better (split_frames)
-    const int64_t n32 = p.algorithm == kExact    ? split_frames<kExact>(p.K, p.nframes)
-                        : p.algorithm == kLinear ? split_frames<kLinear>(p.K, p.nframes)
-                                                 : split_frames<kApproximate>(p.K, p.nframes);
-    if (n32 > 0) {
-      TurboLteParams a = p;
-      a.nframes = n32;
-      a.seg_len = LteGeometry(p.K, 32).seg_len;
-      const size_t smem32 = lte_smem_bytes<32>(p.K);
-      auto run = [&](auto k32, auto k64) -> cudaError_t {
-        cudaError_t err = cudaFuncSetAttribute(k32, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem32));
-        if (err != cudaSuccess) return err;
-        k32<<<unsigned(n32), 64, smem32, s>>>(a);
-        if ((err = cudaGetLastError()) != cudaSuccess) return err;
-        TurboLteParams b = p;
-        b.frame0 = n32;
-        if ((err = cudaFuncSetAttribute(k64, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
-          return err;
-        k64<<<unsigned(p.nframes - n32), 128, smem, s>>>(b);
-        return cudaGetLastError();
-      };
-      switch (p.algorithm) {
-        case kExact: return run(turbo_lte_kernel<kExact, 32>, turbo_lte_kernel<kExact, 64>);
-        case kLinear: return run(turbo_lte_kernel<kLinear, 32>, turbo_lte_kernel<kLinear, 64>);
-        default: return run(turbo_lte_kernel<kApproximate, 32>, turbo_lte_kernel<kApproximate, 64>);
-      }
-    }
-  }
-  switch (p.algorithm) {
-    case kExact: return launch(turbo_lte_kernel<kExact, 64>, 128, smem);
-    case kLinear: return launch(turbo_lte_kernel<kLinear, 64>, 128, smem);
-    default: return launch(turbo_lte_kernel<kApproximate, 64>, 128, smem);
-  }
+  return decode(n32, p.nframes - n32, 64, pick(S64{}, std::false_type{}), lte_smem_bytes<64>(p.K));
+}
+
+// The mixed-K kernel for the algorithm and, in max-log, for batches whose K are all
+// multiples of 8.
+static void (*batch_kernel(int algorithm, bool whole))(TurboLteBatchParams) {
+  if (algorithm == kExact) return turbo_lte_batch_kernel<kExact, kDefaultSegs, true>;
+  if (algorithm == kLinear) return turbo_lte_batch_kernel<kLinear, kDefaultSegs, true>;
+  if (whole) return turbo_lte_batch_kernel<kApproximate, kDefaultSegs, true>;
+  return turbo_lte_batch_kernel<kApproximate, kDefaultSegs, false>;
 }
 
 size_t turbo_lte_frame_floats(int K) { return size_t(LteGeometry(K, kDefaultSegs).frame_floats()); }
 
-int turbo_lte_batch_max_ctas(int max_K, int algorithm) {
+int turbo_lte_batch_max_ctas(int max_K, int algorithm, bool whole) {
   const size_t smem = lte_smem_bytes<kDefaultSegs>(max_K);
   int per_sm = 0, sms = 0, dev = 0;
-  auto q = [&](auto kern) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 2 * kDefaultSegs, smem) != cudaSuccess) {
-      cudaGetLastError();
-      per_sm = 0;
-    }
-  };
-  switch (algorithm) {
-    case kExact: q(turbo_lte_batch_kernel<kExact, kDefaultSegs>); break;
-    case kLinear: q(turbo_lte_batch_kernel<kLinear, kDefaultSegs>); break;
-    default: q(turbo_lte_batch_kernel<kApproximate, kDefaultSegs>); break;
+  auto kern = batch_kernel(algorithm, whole);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 2 * kDefaultSegs, smem) != cudaSuccess) {
+    cudaGetLastError();
+    per_sm = 0;
   }
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     cudaGetLastError();
@@ -1231,20 +1336,14 @@ cudaError_t launch_turbo_lte_batch(const TurboLteBatchParams& p, cudaStream_t s)
   const unsigned stage_blocks = unsigned(q.nframes < 148 * 8 ? q.nframes : 148 * 8);
   turbo_lte_batch_stage<<<stage_blocks, 256, 0, s>>>(q);
   const size_t smem = lte_smem_bytes<kDefaultSegs>(q.max_K);
-  int ctas = q.ctas > 0 ? q.ctas : turbo_lte_batch_max_ctas(q.max_K, q.algorithm);
+  int ctas = q.ctas > 0 ? q.ctas : turbo_lte_batch_max_ctas(q.max_K, q.algorithm, q.whole != 0);
   if (ctas <= 0) return cudaErrorInvalidConfiguration;
   if (int64_t(ctas) > q.nframes) ctas = int(q.nframes);
-  auto launch = [&](auto kern) -> cudaError_t {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (err != cudaSuccess) return err;
-    kern<<<unsigned(ctas), 2 * kDefaultSegs, smem, s>>>(q);
-    return cudaGetLastError();
-  };
-  switch (q.algorithm) {
-    case kExact: return launch(turbo_lte_batch_kernel<kExact, kDefaultSegs>);
-    case kLinear: return launch(turbo_lte_batch_kernel<kLinear, kDefaultSegs>);
-    default: return launch(turbo_lte_batch_kernel<kApproximate, kDefaultSegs>);
-  }
+  auto kern = batch_kernel(q.algorithm, q.whole != 0);
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e != cudaSuccess) return e;
+  kern<<<unsigned(ctas), 2 * kDefaultSegs, smem, s>>>(q);
+  return cudaGetLastError();
 }
 
 }  // namespace fecl

@@ -28,7 +28,10 @@ void set_last_error(const std::string& msg);  // capi.cu
 namespace {
 
 constexpr uint32_t kMaxK = 6144;                       // largest LTE block size
-constexpr size_t kScratchBytes = size_t(8) << 20;      // 8 MiB of scratch per device
+constexpr size_t kAdmitBytes = size_t(8) << 20;        // a call's L-values and checkpoints in time order
+// the same frames in the decoder's slot order (turbo_lte_scratch_bytes), at most 9.94 MiB
+// over the LTE block sizes (7943 frames of K = 40)
+constexpr size_t kScratchBytes = size_t(10) << 20;
 constexpr uint32_t kMaxIterations = 64;
 constexpr uint32_t kPermStride = kMaxK + 16;           // padded for 8-entry vector loads
 constexpr int kMaxDevices = 64;
@@ -75,11 +78,12 @@ extern "C" int fecl_lte_turbo_decode_noalloc(uint32_t K, int32_t algorithm, uint
   if (!llr || !msg) return fail(FECL_EINVAL, "null buffer");
   // The frame count is compared with the capacity before any multiplication, so no
   // count, however large, can wrap the byte size into range.
-  const size_t per_frame = fecl::turbo_lte_scratch_bytes(int(K), 1);
-  const uint64_t max_frames = kScratchBytes / per_frame;
-  if (nframes > max_frames)
+  const size_t chunks = (K + 3 + 7) / 8;  // three arrays of L-values, 8 tail values, two of checkpoints
+  const size_t per_frame = (3 * 8 * chunks + 8 + 2 * 8 * (chunks + 1)) * sizeof(float);
+  const uint64_t max_frames = kAdmitBytes / per_frame;
+  if (nframes > max_frames || fecl::turbo_lte_scratch_bytes(int(K), int64_t(nframes)) > kScratchBytes)
     return fail(FECL_EINVAL, std::to_string(nframes) + " frames of K=" + std::to_string(K) + " need more than the " +
-                                 std::to_string(kScratchBytes) + " bytes of scratch reserved; at most " +
+                                 std::to_string(kAdmitBytes) + " bytes of scratch reserved; at most " +
                                  std::to_string(max_frames) + " frames of K=" + std::to_string(K) + " per call");
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

@@ -316,6 +316,7 @@ bool fecl_server_s::launch(Slot& s, std::vector<std::shared_ptr<Request>>& batch
     p.counter = reinterpret_cast<int32_t*>(base + tdev_off[kv.first].second);
     p.max_K = kv.second.front().K;
     p.algorithm = kv.first;
+    p.whole = std::all_of(kv.second.begin(), kv.second.end(), [](const fecl::TurboLteBatchFrame& t) { return t.K % 8 == 0; });
     cuda_check(fecl::launch_turbo_lte_batch(p, s.stream), "turbo batch launch");
   }
   bool used[kSideStreams] = {};

@@ -365,10 +365,10 @@ int fecl_turbo_window_stats(fecl_codec_t codec, uint64_t* passes, uint64_t* fixu
  * LTE turbo frames (the code of fecl_turbo_create_lte, Serial scheduling, scaling
  * 1.0) with the windowed kernel of fecl_decode, bit-identical to it, but calls no
  * cudaMalloc, cudaFree or allocating library routine.  Its scratch, interleaver and
- * scaling tables are fixed-size static device arrays (8 MiB of scratch, K <= 6144,
+ * scaling tables are fixed-size static device arrays (10 MiB of scratch, K <= 6144,
  * iterations <= 64) that every GPU loading the library holds until process exit;
- * a batch needing more scratch than 8 MiB (more than 68 frames at K = 6144) is
- * rejected with FECL_EINVAL.  llr ([nframes][3K+12]) and msg ([nframes][K] bytes)
+ * a batch whose L-values and checkpoints take more than 8 MiB (more than 68 frames at
+ * K = 6144) is rejected with FECL_EINVAL.  llr ([nframes][3K+12]) and msg ([nframes][K] bytes)
  * are device memory of the current device; the call is asynchronous on `stream`.
  * The first call on a device looks up the arrays' device addresses there, so make
  * it once with each device current before relying on the call being cheap.  All
