@@ -267,7 +267,8 @@ struct TurboLteParams {
   int32_t out_dtype = 1;
   // filled by the launcher
   int32_t Kp = 0, Tp = 0, seg_len = 0, segments = 0, seg_stride = 0, slots = 0;
-  uint4* perm_pos = nullptr;  // [slots] interleaved positions
+  uint4* perm_pos = nullptr;  // [slots] interleaved positions (stage_here: of every frame)
+  int32_t stage_here = 0;     // the decoding CTAs stage their frames
   int64_t frame0 = 0;  // frame of the launch's first CTA
   int64_t frame_stride = 0;
   float* ck = nullptr;

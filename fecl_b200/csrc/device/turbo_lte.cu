@@ -339,14 +339,16 @@ __device__ __forceinline__ float par_step(const float a[8], const float b[8], co
 // array holds its chunks by k and then by w: chunk c = w Lc + k at slot k Sp + w, as two
 // planes of 4 floats per slot.  A warp's load of one plane is then contiguous (with the
 // chunks in time order it touched one line per lane, and the L1 pipe, at 73 % of its
-// peak, bound the kernel).  The exchange arrays in shared memory hold step t at
-// (t mod 8) nblk + t / 8: neighbouring chunks fall into neighbouring banks, and so do, for
-// an odd number of chunks per segment, the interleaved positions, since a QPP interleaver
-// maps steps that differ by a multiple of 8 to positions that do.
+// peak, bound the kernel).  The exchange arrays in shared memory are in time order with the
+// halves of every other group of 4 chunks swapped: a chunk is two 16-byte accesses, which
+// for an odd number of chunks per segment fall into distinct banks over the lanes, and
+// interleaved positions (a QPP interleaver maps steps that differ by a multiple of 8 to
+// positions that do) into 8 banks instead of 4.  One plane per step modulo 8 had no
+// conflicts at all, but took 13 instructions more per chunk, and instructions bound the kernel.
 struct LteMap {
   int Lc, S, Sp, slots, nblk;
   __device__ __forceinline__ int slot_of(int c) const { return (c % Lc) * Sp + c / Lc; }
-  __device__ __forceinline__ int pos(int t) const { return (t & 7) * nblk + (t >> 3); }
+  __device__ __forceinline__ static int pos(int t) { return t ^ ((t >> 3) & 4); }
 };
 
 struct Frame {
@@ -355,7 +357,7 @@ struct Frame {
   const float* Lp0;   // [2][slots][4] parity (with tail parity) of constituent 0
   const float* Lp1;   // [2][slots][4]
   const float* ts;    // [8]  tail systematic of constituent 0 (3) then 1 (3)
-  const uint4* perm;  // [slots] position of each step's interleaved index, 16 bits each
+  const uint4* perm;  // [slots] byte offset of each step's interleaved element, 16 bits each
   float* cka;         // [2][slots][4] forward metrics before each chunk
   float* ckb;         // [2][slots][4] backward metrics before each chunk (chunk nblk: the end)
 };
@@ -378,23 +380,27 @@ struct RawChunk {
 };
 
 __device__ __forceinline__ void load_raw(int j, int slot, const Frame& fr, RawChunk& r) {
+  // plain loads: a small batch's CTAs stage their frames themselves
   const float4* Lp = reinterpret_cast<const float4*>(j == 0 ? fr.Lp0 : fr.Lp1) + slot;
-  r.p0 = __ldg(Lp);
-  r.p1 = __ldg(Lp + fr.m.slots);
+  r.p0 = Lp[0];
+  r.p1 = Lp[fr.m.slots];
   if (j == 0) {
     const uint4* q = reinterpret_cast<const uint4*>(fr.Ls) + slot;
-    r.q0 = __ldg(q);
-    r.q1 = __ldg(q + fr.m.slots);
+    r.q0 = q[0];
+    r.q1 = q[fr.m.slots];
   } else {
-    r.q0 = __ldg(fr.perm + slot);
+    r.q0 = fr.perm[slot];
   }
 }
 
-// Entry i of the 8 16-bit positions of a chunk.
-__device__ __forceinline__ uint32_t pos_of(const uint4& q, int i) {
+// Entry i of the 8 16-bit offsets of a chunk.
+__device__ __forceinline__ uint32_t offset_of(const uint4& q, int i) {
   const uint32_t w = i < 2 ? q.x : i < 4 ? q.y : i < 6 ? q.z : q.w;
   return (i & 1) ? w >> 16 : w & 0xffffu;
 }
+
+// The two halves of chunk c in an exchange array (in 4-float units): steps 0 to 3 and 4 to 7.
+__device__ __forceinline__ int half_of(int c, int h) { return 2 * c + (h ^ ((c >> 2) & 1)); }
 
 // A chunk's a-priori and parity L-values.
 struct Chunk {
@@ -402,8 +408,10 @@ struct Chunk {
   float lp[kBlk];
 };
 
-__device__ __forceinline__ void resolve(int j, int c, int K, const Frame& fr, const float* X, const float* Y,
-                                        const RawChunk& r, Chunk& ch) {
+// The CTA's dynamic shared memory; the exchange arrays X and Y start at 0 and at Kp.
+extern __shared__ __align__(16) float lte_smem[];
+
+__device__ __forceinline__ void resolve(int j, int c, int K, const Frame& fr, int Kp, const RawChunk& r, Chunk& ch) {
   const int t0 = c * kBlk;
   ch.lp[0] = r.p0.x; ch.lp[1] = r.p0.y; ch.lp[2] = r.p0.z; ch.lp[3] = r.p0.w;
   ch.lp[4] = r.p1.x; ch.lp[5] = r.p1.y; ch.lp[6] = r.p1.z; ch.lp[7] = r.p1.w;
@@ -411,12 +419,14 @@ __device__ __forceinline__ void resolve(int j, int c, int K, const Frame& fr, co
     const float ls[kBlk] = {__uint_as_float(r.q0.x), __uint_as_float(r.q0.y), __uint_as_float(r.q0.z),
                             __uint_as_float(r.q0.w), __uint_as_float(r.q1.x), __uint_as_float(r.q1.y),
                             __uint_as_float(r.q1.z), __uint_as_float(r.q1.w)};
-    const float* y = Y + c;
+    const float4* y = reinterpret_cast<const float4*>(lte_smem + Kp);
+    const float4 y0 = y[half_of(c, 0)], y1 = y[half_of(c, 1)];
+    const float yv[kBlk] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
 #pragma unroll
-    for (int i = 0; i < kBlk; ++i) ch.la[i] = ls[i] + y[i * fr.m.nblk];
+    for (int i = 0; i < kBlk; ++i) ch.la[i] = ls[i] + yv[i];
   } else {
 #pragma unroll
-    for (int i = 0; i < kBlk; ++i) ch.la[i] = X[pos_of(r.q0, i)];
+    for (int i = 0; i < kBlk; ++i) ch.la[i] = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(lte_smem) + offset_of(r.q0, i));
   }
   if (t0 + kBlk > K) {
 #pragma unroll
@@ -466,8 +476,12 @@ __device__ __forceinline__ bool close8(const float x[8], const float y[8], Tol t
 // checkpoints and end stand.  Kept out of line so that Phase A and the fix-up rounds share
 // one copy of the code.
 template <int ALG>
-__device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float4 va, float4 vb, float* vbound, int segs,
-                                          int K, int T, Frame fr, const float* X, const float* Y, bool refine, Tol tol) {
+__device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float4 va, float4 vb, int bound, int segs,
+                                          int K, int T, Frame fr, int Kp, bool refine, Tol tol) {
+  // out of line, the address spaces are not known
+  __builtin_assume(__isGlobal(fr.Ls) && __isGlobal(fr.Lp0) && __isGlobal(fr.Lp1) && __isGlobal(fr.ts));
+  __builtin_assume(__isGlobal(fr.perm) && __isGlobal(fr.cka) && __isGlobal(fr.ckb));
+  float* vbound = lte_smem + bound;
   float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
   const int Lc = fr.m.Lc, Sp = fr.m.Sp, slots = fr.m.slots, nblk = fr.m.nblk;
   const int turn = (Lc - 1) * Sp - 1;  // from a segment's last slot back to the next one's first
@@ -479,8 +493,8 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float
     RawChunk nxt;
     load_raw(j, slot, fr, nxt);
     for (; c < c_end; ++c) {
-      const RawChunk cur = nxt;
       const int here = slot;
+      const RawChunk cur = nxt;
       if (++kk == Lc) {
         kk = 0;
         slot -= turn;
@@ -488,6 +502,8 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float
         slot += Sp;
       }
       if (c + 1 < c_end) load_raw(j, slot, fr, nxt);
+      Chunk ch;
+      resolve(j, c, K, fr, Kp, cur, ch);
       if (c >= c_own) {
         if (refine && c > c_own) {
           float old[8];
@@ -496,8 +512,6 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float
         }
         store_ck(fr.cka, slots, here, v);
       }
-      Chunk ch;
-      resolve(j, c, K, fr, X, Y, cur, ch);
       const int n = min(kBlk, T - c * kBlk);
       if (n == kBlk) {  // every chunk but the frame's last, whose few steps run in a loop
 #pragma unroll
@@ -534,8 +548,8 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float
     RawChunk nxt;
     load_raw(j, slot, fr, nxt);
     for (; c >= c_own; --c) {
-      const RawChunk cur = nxt;
       const int here = slot;
+      const RawChunk cur = nxt;
       if (--kk < 0) {
         kk = Lc - 1;
         slot += turn;
@@ -544,7 +558,7 @@ __device__ __noinline__ void segment_walk(int fwd, int j, int w, int lead, float
       }
       if (c > c_own) load_raw(j, slot, fr, nxt);
       Chunk ch;
-      resolve(j, c, K, fr, X, Y, cur, ch);
+      resolve(j, c, K, fr, Kp, cur, ch);
       const int hi = min(kBlk, T - c * kBlk);
       if (hi == kBlk) {  // as in the forward walk
 #pragma unroll
@@ -603,8 +617,7 @@ struct SoftSink {
 // soDecode's last iteration, which also records every step's extrinsic value (tail
 // steps too) and parity extrinsic value in `sink`.
 template <int ALG, bool FULL, bool SOFT>
-__device__ __forceinline__ void ext_block(int j, int k, int w, int K, int T, const Frame& fr, const float* X,
-                                          const float* Y, float sf, float* out, const SoftSink& sink) {
+__device__ __forceinline__ void ext_block(int j, int k, int w, int K, int T, const Frame& fr, int Kp, float sf, float* out, const SoftSink& sink) {
   const int b = w * fr.m.Lc + k, slot = k * fr.m.Sp + w, slots = fr.m.slots;
   const int after = k + 1 < fr.m.Lc ? slot + fr.m.Sp : w + 1;  // chunk b + 1
   const int t0 = b * kBlk;
@@ -616,7 +629,7 @@ __device__ __forceinline__ void ext_block(int j, int k, int w, int K, int T, con
   float be[8];
   load_ck(fr.ckb, slots, after, be);
   Chunk in;
-  resolve(j, b, K, fr, X, Y, raw, in);
+  resolve(j, b, K, fr, Kp, raw, in);
 #pragma unroll
   for (int i = 1; i < kBlk; ++i) {
     if (FULL || i < n) {
@@ -630,15 +643,17 @@ __device__ __forceinline__ void ext_block(int j, int k, int w, int K, int T, con
   const float ls[kBlk] = {__uint_as_float(raw.q0.x), __uint_as_float(raw.q0.y), __uint_as_float(raw.q0.z),
                           __uint_as_float(raw.q0.w), __uint_as_float(raw.q1.x), __uint_as_float(raw.q1.y),
                           __uint_as_float(raw.q1.z), __uint_as_float(raw.q1.w)};
+  float x[kBlk] = {};
 #pragma unroll
   for (int i = kBlk - 1; i >= 0; --i) {
     if (FULL || i < n) {
       Gam g;
       g.set(in.la[i], in.lp[i]);
       const float e = sf * ext_step<ALG>(al[i], be, g);
-      if (FULL || t0 + i < K) {
-        if (j == 0) out[i * fr.m.nblk + b] = ls[i] + e;
-        else out[pos_of(raw.q0, i)] = e;
+      if (FULL && j == 0) x[i] = ls[i] + e;
+      else if (FULL || t0 + i < K) {
+        if (j == 0) out[fr.m.pos(t0 + i)] = ls[i] + e;
+        else *reinterpret_cast<float*>(reinterpret_cast<char*>(out) + offset_of(raw.q0, i)) = e;
       }
       if (SOFT && sink.ext) {
         sink.ext[t0 + i] = e;
@@ -647,14 +662,18 @@ __device__ __forceinline__ void ext_block(int j, int k, int w, int K, int T, con
       if (i > 0) bwd_step<ALG>(be, g);
     }
   }
+  if (FULL && j == 0) {
+    float4* o = reinterpret_cast<float4*>(out);
+    o[half_of(b, 0)] = make_float4(x[0], x[1], x[2], x[3]);
+    o[half_of(b, 1)] = make_float4(x[4], x[5], x[6], x[7]);
+  }
 }
 
 // The same block for the log-MAP algorithms, step by step: their steps are long (dozens of
 // instructions per log-sum), and 8 of them unrolled three times over ran from the
 // instruction cache's misses.  The forward vectors wait in local memory.
 template <int ALG, bool SOFT>
-__device__ __forceinline__ void ext_steps(int j, int k, int w, int K, int T, const Frame& fr, const float* X, const float* Y,
-                                          float sf, float* out, const SoftSink& sink) {
+__device__ __forceinline__ void ext_steps(int j, int k, int w, int K, int T, const Frame& fr, int Kp, float sf, float* out, const SoftSink& sink) {
   const int b = w * fr.m.Lc + k, slot = k * fr.m.Sp + w, slots = fr.m.slots;
   const int after = k + 1 < fr.m.Lc ? slot + fr.m.Sp : w + 1;  // chunk b + 1
   const int t0 = b * kBlk, n = min(kBlk, T - t0);
@@ -664,7 +683,7 @@ __device__ __forceinline__ void ext_steps(int j, int k, int w, int K, int T, con
   load_ck(fr.cka, slots, slot, v);
   load_ck(fr.ckb, slots, after, be);
   Chunk in;
-  resolve(j, b, K, fr, X, Y, raw, in);
+  resolve(j, b, K, fr, Kp, raw, in);
   float4 al[kBlk][2];
 #pragma unroll 1
   for (int i = 0;; ++i) {
@@ -684,8 +703,8 @@ __device__ __forceinline__ void ext_steps(int j, int k, int w, int K, int T, con
     g.set(in.la[i], in.lp[i]);
     const float e = sf * ext_step<ALG>(a, be, g);
     if (t0 + i < K) {
-      if (j == 0) out[i * fr.m.nblk + b] = __uint_as_float(q[i]) + e;
-      else out[(i & 1) ? q[i >> 1] >> 16 : q[i >> 1] & 0xffffu] = e;
+      if (j == 0) out[fr.m.pos(t0 + i)] = __uint_as_float(q[i]) + e;
+      else *reinterpret_cast<float*>(reinterpret_cast<char*>(out) + ((i & 1) ? q[i >> 1] >> 16 : q[i >> 1] & 0xffffu)) = e;
     }
     if (SOFT && sink.ext) {
       sink.ext[t0 + i] = e;
@@ -741,20 +760,20 @@ __host__ __device__ inline int lte_seg_len(int T, int segs) {
   return (L + kBlk - 1) / kBlk * kBlk;
 }
 
-// Decodes one frame with the whole CTA; smem holds 2 * Kp floats + Shared<SEGS>.
+// Decodes one frame with the whole CTA; lte_smem holds 2 * Kp floats + Shared<SEGS>.
 // SOFT: soDecode (TurboDecoderImpl::soDecodeBlock, TurboDecoderImpl.cpp:75-150).
 // WHOLE: K is a multiple of 8, as every LTE size is (the max-log kernels have a form for each,
 // so that none carries both: their code has to stay in the instruction cache).
 template <int ALG, int SEGS, bool SOFT, bool WHOLE>
-__device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
+__device__ __forceinline__ void decode_lte_frame(const LteJob& q) {
   constexpr int kThreads = 2 * SEGS;
   const int K = q.K, T = q.K + 3;
   const LteMap& m = q.map;
   const int nblk = m.nblk;
   const int nblk_msg = (K + kBlk - 1) / kBlk;
-  float* X = smem;
-  float* Y = smem + q.Kp;
-  Shared<SEGS>& sh = *reinterpret_cast<Shared<SEGS>*>(smem + 2 * q.Kp);
+  float* X = lte_smem;
+  float* Y = lte_smem + q.Kp;
+  Shared<SEGS>& sh = *reinterpret_cast<Shared<SEGS>*>(lte_smem + 2 * q.Kp);
   Frame fr;
   fr.m = m;
   fr.Ls = q.scratch;
@@ -773,12 +792,11 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
   for (int i = tid; i < nblk; i += kThreads) {
     int k, w;
     block_at(i, nblk, m, k, w);
-    float l[8];
-    load_ck(fr.Ls, m.slots, k * m.Sp + w, l);
+    const float4* l = reinterpret_cast<const float4*>(fr.Ls) + k * m.Sp + w;
 #pragma unroll
-    for (int u = 0; u < kBlk; ++u) {
-      X[u * nblk + w * Lc + k] = l[u];
-      Y[u * nblk + w * Lc + k] = 0.0f;
+    for (int h = 0; h < 2; ++h) {
+      reinterpret_cast<float4*>(X)[half_of(w * Lc + k, h)] = l[h * m.slots];
+      reinterpret_cast<float4*>(Y)[half_of(w * Lc + k, h)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
   // Tail: the trellis starts and ends in state 0; training starts from all states equal
@@ -793,7 +811,7 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
     const uint16_t* perm = reinterpret_cast<const uint16_t*>(fr.perm);
     for (int k = tid; k < K; k += kThreads) {
       X[m.pos(k)] = X[m.pos(k)] + load_llr(q.state_in, q.in_dtype, s0 + k);
-      Y[perm[m.slot_of(k >> 3) * 8 + (k & 7)]] = load_llr(q.state_in, q.in_dtype, s0 + K + 3 + k);
+      Y[perm[m.slot_of(k >> 3) * 8 + (k & 7)] / 4] = load_llr(q.state_in, q.in_dtype, s0 + K + 3 + k);
     }
     __syncthreads();
   }
@@ -801,6 +819,7 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
   int ran = q.iterations;
   for (int it = 0; it < q.iterations; ++it) {
     const bool last_soft = SOFT && it == q.iterations - 1;
+#pragma unroll 1
     for (int jj = 0; jj < 2; ++jj) {
       const int j = q.parallel ? 1 - jj : jj;  // parallel: constituent 1 first, on the old X
       const bool fwd = tid < SEGS;
@@ -813,7 +832,7 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
         // a forward start is the checkpoint at a0, a backward end the one at a0
         if (w < S)
           segment_walk<ALG>(fwd, j, w, lead, exact ? term_a : flat, exact ? term_b : flat,
-                            fwd ? &sh.fwd_end[0][0] : &sh.bwd_start[0][0], SEGS, K, T, fr, X, Y, false, tol);
+                            int((fwd ? &sh.fwd_end[0][0] : &sh.bwd_start[0][0]) - lte_smem), SEGS, K, T, fr, q.Kp, false, tol);
       }
       __syncthreads();
       // ---- A2: verify boundaries; walk again the segments whose start disagrees.
@@ -848,7 +867,7 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
           if (q.stats) atomicAdd(q.stats + 2, 1ull);
           segment_walk<ALG>(fwd, j, w, 0, make_float4(right[0], right[1], right[2], right[3]),
                             make_float4(right[4], right[5], right[6], right[7]),
-                            fwd ? &sh.fwd_end[0][0] : &sh.bwd_start[0][0], SEGS, K, T, fr, X, Y, true, tol);
+                            int((fwd ? &sh.fwd_end[0][0] : &sh.bwd_start[0][0]) - lte_smem), SEGS, K, T, fr, q.Kp, true, tol);
         }
         __syncthreads();
       }
@@ -877,8 +896,8 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
         int kb, wb;
         block_at(i, blocks, m, kb, wb);
         // WHOLE: every message block has 8 message steps, and runs without per-step tests
-        if constexpr (ALG == kApproximate) ext_block<ALG, WHOLE && !SOFT, SOFT>(j, kb, wb, K, T, fr, X, Y, sf, out, sink);
-        else ext_steps<ALG, SOFT>(j, kb, wb, K, T, fr, X, Y, sf, out, sink);
+        if constexpr (ALG == kApproximate) ext_block<ALG, WHOLE && !SOFT, SOFT>(j, kb, wb, K, T, fr, q.Kp, sf, out, sink);
+        else ext_steps<ALG, SOFT>(j, kb, wb, K, T, fr, q.Kp, sf, out, sink);
       }
       __syncthreads();
     }
@@ -891,6 +910,7 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
     // K decided bits is the xor of the table entries of the bits that are 1.
     if (q.crc) {
       uint32_t syn = 0;
+#pragma unroll 1
       for (int k = tid; k < K; k += kThreads)
         if ((X[m.pos(k)] + Y[m.pos(k)]) > 0.0f) syn ^= __ldg(q.crc + k);
 #pragma unroll
@@ -934,25 +954,128 @@ __device__ __forceinline__ void decode_lte_frame(const LteJob& q, float* smem) {
   } else {
     // a-posteriori and hard decision, TurboDecoderImpl.cpp:64-71
     if (K % 8 == 0 && reinterpret_cast<uintptr_t>(q.hard) % 8 == 0) {
+#pragma unroll 1
       for (int b = tid; b < K / 8; b += kThreads) {
-        uint32_t lo = 0, hi = 0;
+        uint32_t bits[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          lo |= uint32_t((X[i * nblk + b] + Y[i * nblk + b]) > 0.0f) << (8 * i);
-          hi |= uint32_t((X[(i + 4) * nblk + b] + Y[(i + 4) * nblk + b]) > 0.0f) << (8 * i);
+        for (int h = 0; h < 2; ++h) {
+          const float4 x = reinterpret_cast<const float4*>(X)[half_of(b, h)], y = reinterpret_cast<const float4*>(Y)[half_of(b, h)];
+          bits[h] = uint32_t((x.x + y.x) > 0.0f) | uint32_t((x.y + y.y) > 0.0f) << 8 | uint32_t((x.z + y.z) > 0.0f) << 16 |
+                    uint32_t((x.w + y.w) > 0.0f) << 24;
         }
-        reinterpret_cast<uint2*>(q.hard)[b] = make_uint2(lo, hi);
+        reinterpret_cast<uint2*>(q.hard)[b] = make_uint2(bits[0], bits[1]);
       }
     } else {
+#pragma unroll 1
       for (int k = tid; k < K; k += kThreads) q.hard[k] = uint8_t((X[m.pos(k)] + Y[m.pos(k)]) > 0.0f);
     }
     if (q.iters && tid == 0) *q.iters = ran;
   }
 }
 
+template <typename T>
+__device__ __forceinline__ float to_f32(T v) { return float(v); }
+template <>
+__device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
+
+// Slots of chunks with the quotient by Lc (chunk numbers below 2^11) as a multiplication.
+struct SlotOf {
+  int Lc, Sp, plane;
+  uint32_t inv;
+  __device__ __forceinline__ explicit SlotOf(const LteMap& m)
+      : Lc(m.Lc), Sp(m.Sp), plane(4 * m.slots), inv(m.Lc > 1 ? 0xffffffffu / uint32_t(m.Lc) + 1u : 0u) {}
+  __device__ __forceinline__ int slot(int c) const {
+    if (Lc == 1) return c;
+    const int w = int(__umulhi(uint32_t(c), inv));
+    return (c - w * Lc) * Sp + w;
+  }
+  // where step t's element of a staged array lies
+  __device__ __forceinline__ int element(int t) const { return ((t >> 2) & 1) * plane + slot(t >> 3) * 4 + (t & 3); }
+};
+
+// One frame's input [3K+12] in FeCl's turbo layout | msg [K] | systTail1 [3] | systTail2 [3] |
+// parity1 [K+3] | parity2 [K+3] | -> FP32 scratch in slot order: the regions are copied by
+// loops of their own, and the element type is fixed per launch.  soDecode's a-priori input is added
+// to the channel's systematic values and tails (TurboDecoderImpl.cpp:77-82).
+template <typename T>
+__device__ __forceinline__ void stage_frame(const T* in, const T* sys, float* out, int K, int Tp, const LteMap& m) {
+  const SlotOf where(m);
+  // four elements per thread and step, all loaded before any is stored, so that each
+  // thread keeps four loads in flight (load latency, not bandwidth, bounds the copy)
+  constexpr int kU = 4;
+  const int step = int(blockDim.x);
+  for (int i0 = threadIdx.x; i0 < Tp; i0 += kU * step) {
+    float v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int i = i0 + u * step;
+      v[u] = i < K ? (sys ? to_f32(in[i]) + to_f32(sys[i]) : to_f32(in[i])) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (i0 + u * step < Tp) out[where.element(i0 + u * step)] = v[u];
+  }
+  for (int c = 0; c < 2; ++c) {
+    const T* src = in + K + 6 + c * (K + 3);  // parity (with its tail) of constituent c
+    float* dst = out + (1 + c) * 8 * m.slots;
+    for (int t0 = threadIdx.x; t0 < Tp; t0 += kU * step) {
+      float v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int t = t0 + u * step;
+        v[u] = t < K + 3 ? to_f32(src[t]) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (t0 + u * step < Tp) dst[where.element(t0 + u * step)] = v[u];
+    }
+  }
+  if (threadIdx.x < 8) {
+    float v = 0.0f;
+    if (threadIdx.x < 6) v = sys ? to_f32(in[K + threadIdx.x]) + to_f32(sys[K + threadIdx.x]) : to_f32(in[K + threadIdx.x]);
+    out[24 * m.slots + threadIdx.x] = v;
+  }
+}
+
+// The byte offset of every step's interleaved element (LteMap::pos; K <= 12288: 16 bits), in
+// slot order; steps past K read the first.
+__device__ __forceinline__ void stage_positions(const uint32_t* perm, uint16_t* out, int K, int Tp, const LteMap& m,
+                                                int first, int step) {
+  const SlotOf where(m);
+#pragma unroll 4
+  for (int t = first; t < Tp; t += step) out[where.slot(t >> 3) * 8 + (t & 7)] = t < K ? uint16_t(4 * m.pos(int(__ldg(perm + t)))) : 0;
+}
+
+// A CTA's own staging of its frame and of positions for it alone (launches of at most one frame
+// per SM, which this saves the staging launch).
+__device__ __noinline__ void stage_here(const TurboLteParams& p, int64_t f, float* out, uint16_t* positions, LteMap m) {
+  const int K = p.K;
+  const int64_t in0 = f * int64_t(3 * K + 12), sys0 = f * int64_t(K + 6);
+  const SlotOf where(m);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < 3 * p.Tp; i += blockDim.x) {
+    const int c = i < p.Tp ? 0 : i < 2 * p.Tp ? 1 : 2, t = i - c * p.Tp;  // systematic, parity 1, parity 2
+    float v = 0.0f;
+    if (t < (c ? K + 3 : K)) {
+      v = load_llr(p.llr, p.llr_dtype, size_t(in0 + (c ? K + 6 + (c - 1) * (K + 3) : 0) + t));
+      if (c == 0 && p.syst_in) v += load_llr(p.syst_in, p.llr_dtype, size_t(sys0 + t));
+    }
+    out[c * 8 * m.slots + where.element(t)] = v;
+  }
+  if (threadIdx.x < 8) {
+    float v = 0.0f;
+    if (threadIdx.x < 6) {
+      v = load_llr(p.llr, p.llr_dtype, size_t(in0 + K + threadIdx.x));
+      if (p.syst_in) v += load_llr(p.syst_in, p.llr_dtype, size_t(sys0 + K + threadIdx.x));
+    }
+    out[24 * m.slots + threadIdx.x] = v;
+  }
+  stage_positions(p.perm[1], positions, K, p.Tp, m, threadIdx.x, blockDim.x);
+  __syncthreads();
+}
+
 template <int ALG, int SEGS, bool SOFT, bool WHOLE>
-__global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : (SEGS == 128 ? 1 : 3)) turbo_lte_kernel(TurboLteParams p) {
-  extern __shared__ float smem[];
+__global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : (SEGS == 128 ? 1 : 3)) turbo_lte_kernel(const __grid_constant__ TurboLteParams p) {
   const int64_t f = p.frame0 + blockIdx.x;
   LteJob q;
   q.K = p.K;
@@ -964,6 +1087,11 @@ __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : (SEGS == 128 ? 1 : 
   q.sf = p.sf;
   q.perm = p.perm_pos;
   q.scratch = p.scratch + int64_t(blockIdx.x) * p.frame_stride;
+  if (p.stage_here) {
+    q.perm = p.perm_pos + int64_t(blockIdx.x) * p.slots;
+    stage_here(p, f, p.scratch + int64_t(blockIdx.x) * p.frame_stride,
+               reinterpret_cast<uint16_t*>(p.perm_pos + int64_t(blockIdx.x) * p.slots), q.map);
+  }
   q.ck = p.ck + int64_t(blockIdx.x) * (16 * p.slots);
   q.hard = p.hard + f * p.K;
   q.iters = p.iters ? p.iters + f : nullptr;
@@ -982,14 +1110,9 @@ __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : (SEGS == 128 ? 1 : 
   q.parity_out = p.parity_out;
   q.state_out = p.state_out;
   q.frame = f;
-  decode_lte_frame<ALG, SEGS, SOFT, WHOLE>(q, smem);
+  decode_lte_frame<ALG, SEGS, SOFT, WHOLE>(q);
 }
 
-
-template <typename T>
-__device__ __forceinline__ float to_f32(T v) { return float(v); }
-template <>
-__device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
 
 // Geometry of a frame of K message bits: T trellis steps, nblk 8-step chunks, the padded
 // length Kp = Tp of the exchange arrays, and the staged layout of `segs` forward and `segs`
@@ -1015,69 +1138,6 @@ struct LteGeometry {
   // bytes so frames share no cache line.
   __host__ __device__ int frame_floats() const { return (staged_floats() + ck_floats() + perm_floats() + 31) & ~31; }
 };
-
-// Quotients by Lc of chunk numbers (below 2^11) as a multiplication.
-__device__ __forceinline__ int staged_at(int t, const LteMap& m, uint32_t inv) {
-  const int c = t >> 3, w = int(__umulhi(uint32_t(c), inv)), slot = (c - w * m.Lc) * m.Sp + w;
-  return ((t >> 2) & 1) * 4 * m.slots + slot * 4 + (t & 3);
-}
-__device__ __forceinline__ uint32_t inverse_of(int d) { return d > 1 ? 0xffffffffu / uint32_t(d) + 1u : 0u; }
-
-// One frame's input [3K+12] in FeCl's turbo layout | msg [K] | systTail1 [3] | systTail2 [3] |
-// parity1 [K+3] | parity2 [K+3] | -> FP32 scratch in slot order: the regions are copied by
-// loops of their own, and the element type is fixed per launch.  soDecode's a-priori input is added
-// to the channel's systematic values and tails (TurboDecoderImpl.cpp:77-82).  Lc = 1 has
-// no quotient: chunk c is segment c.
-template <typename T>
-__device__ __forceinline__ void stage_frame(const T* in, const T* sys, float* out, int K, int Tp, const LteMap& m) {
-  const uint32_t inv = inverse_of(m.Lc);
-  auto at = [&](int t) {
-    if (m.Lc == 1) return ((t >> 2) & 1) * 4 * m.slots + (t >> 3) * 4 + (t & 3);
-    return staged_at(t, m, inv);
-  };
-  // four elements per thread and step, all loaded before any is stored, so that each
-  // thread keeps four loads in flight (load latency, not bandwidth, bounds the copy)
-  constexpr int kU = 4;
-  const int step = int(blockDim.x);
-  for (int i0 = threadIdx.x; i0 < Tp; i0 += kU * step) {
-    float v[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int i = i0 + u * step;
-      v[u] = i < K ? (sys ? to_f32(in[i]) + to_f32(sys[i]) : to_f32(in[i])) : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (i0 + u * step < Tp) out[at(i0 + u * step)] = v[u];
-  }
-  for (int c = 0; c < 2; ++c) {
-    const T* src = in + K + 6 + c * (K + 3);  // parity (with its tail) of constituent c
-    float* dst = out + (1 + c) * 8 * m.slots;
-    for (int t0 = threadIdx.x; t0 < Tp; t0 += kU * step) {
-      float v[kU];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int t = t0 + u * step;
-        v[u] = t < K + 3 ? to_f32(src[t]) : 0.0f;
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u)
-        if (t0 + u * step < Tp) dst[at(t0 + u * step)] = v[u];
-    }
-  }
-  if (threadIdx.x < 8) {
-    float v = 0.0f;
-    if (threadIdx.x < 6) v = sys ? to_f32(in[K + threadIdx.x]) + to_f32(sys[K + threadIdx.x]) : to_f32(in[K + threadIdx.x]);
-    out[24 * m.slots + threadIdx.x] = v;
-  }
-}
-
-// The interleaved position (LteMap::pos) of every step, 16 bits each, in slot order; steps
-// past K read position 0.
-__device__ __forceinline__ void stage_positions(const uint32_t* perm, uint16_t* out, int K, int Tp, const LteMap& m,
-                                                int first, int step) {
-  for (int t = first; t < Tp; t += step) out[m.slot_of(t >> 3) * 8 + (t & 7)] = t < K ? uint16_t(m.pos(int(perm[t]))) : 0;
-}
 
 // Staging of a launch's frames (grid-strided) and, by the last block, of its positions.
 template <typename T>
@@ -1116,7 +1176,6 @@ __global__ void turbo_lte_batch_stage(TurboLteBatchParams p) {
 // and the long ones do not trail behind.  Shared memory is sized for the largest K.
 template <int ALG, int SEGS, bool WHOLE>
 __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : 3) turbo_lte_batch_kernel(TurboLteBatchParams p) {
-  extern __shared__ float smem[];
   __shared__ int next;
   for (;;) {
     __syncthreads();  // every thread has read `next` (and finished the last frame)
@@ -1141,7 +1200,7 @@ __global__ void __launch_bounds__(2 * SEGS, SEGS == 32 ? 4 : 3) turbo_lte_batch_
     q.iters = d.iters;
     q.stats = p.stats;
     q.crc = d.crc;
-    decode_lte_frame<ALG, SEGS, false, WHOLE>(q, smem);
+    decode_lte_frame<ALG, SEGS, false, WHOLE>(q);
   }
 }
 
@@ -1149,6 +1208,9 @@ template <int SEGS>
 size_t lte_smem_bytes(int max_K) {
   return size_t(2 * LteGeometry(max_K, SEGS).Kp) * sizeof(float) + sizeof(Shared<SEGS>);
 }
+
+// Frames that CTAs may stage themselves (one per SM of a 148-SM GPU).
+constexpr int64_t kStageHere = 148;
 
 int resolve_segs(int segs) { return segs == 32 || segs == 64 || segs == 128 ? segs : kDefaultSegs; }
 
@@ -1211,7 +1273,8 @@ cudaError_t turbo_lte_init() {
 }
 
 size_t turbo_lte_scratch_bytes(int K, int64_t nframes, bool extra) {
-  // whichever shapes the launcher takes: the largest frame of the three, and positions for two launches
+  // whichever shapes the launcher takes: the largest frame of the three, and positions for two
+  // launches or for every frame of a small batch
   int frame = 0, positions = 0;
   for (int segs : {32, 64, 128}) {
     const LteGeometry g(K, segs);
@@ -1219,7 +1282,9 @@ size_t turbo_lte_scratch_bytes(int K, int64_t nframes, bool extra) {
     positions = std::max(positions, g.perm_floats());
   }
   const int Tp = LteGeometry(K, kDefaultSegs).Tp;
-  return (size_t(nframes) * (size_t(frame) + (extra ? size_t(3 * Tp) : 0)) + 2 * size_t(positions)) * sizeof(float);
+  return (size_t(nframes) * (size_t(frame) + (extra ? size_t(3 * Tp) : 0)) +
+          size_t(nframes <= kStageHere ? nframes + 1 : 2) * size_t(positions)) *
+         sizeof(float);
 }
 
 cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
@@ -1235,6 +1300,13 @@ cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
   const int sms = device_sms();
   if (p.soft) segs = 64;
   else if (p.segs == 0 && p.nframes <= sms) segs = 128;
+  // Short frames: the fewest threads whose segments are the same (K <= 248: 8 steps each in
+  // every shape; warps without a segment only lengthen the barriers).
+  auto narrowest = [&](int segs) {
+    while (!p.soft && segs > 32 && lte_seg_len(p.K + 3, segs / 2) == lte_seg_len(p.K + 3, segs)) segs /= 2;
+    return segs;
+  };
+  segs = narrowest(segs);
   if (p.soft) p.crc = nullptr;
   if (p.train < 0) p.train = default_train(p.algorithm);
   float* at = p.scratch;
@@ -1259,9 +1331,10 @@ cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
     q.ynew = (p.parallel || p.soft) ? at : nullptr;
     if (q.ynew) at += n * int64_t(3 * g.Tp);
     q.perm_pos = reinterpret_cast<uint4*>(at);
-    at += g.perm_floats();
+    q.stage_here = p.nframes <= kStageHere && p.nframes <= sms;
+    at += (q.stage_here ? n : 1) * int64_t(g.perm_floats());
     const unsigned blocks = unsigned(n < 148 * 8 ? n : 148 * 8) + 1;
-    switch (p.llr_dtype) {
+    if (!q.stage_here) switch (p.llr_dtype) {
       case kF64: turbo_lte_stage<double><<<blocks, 256, 0, s>>>(q); break;
       case kF16: turbo_lte_stage<__half><<<blocks, 256, 0, s>>>(q); break;
       default: turbo_lte_stage<float><<<blocks, 256, 0, s>>>(q); break;
@@ -1289,7 +1362,7 @@ cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
   if (segs == 128) return decode(0, p.nframes, 128, pick(S128{}, std::false_type{}), lte_smem_bytes<128>(p.K));
   // the launcher's choice: whole rounds of the 32-segment shape first where that fills
   // the rounds better (split_frames)
-  const int64_t n32 = p.segs == 0 ? split_frames(p.K, p.nframes, sms) : 0;
+  const int64_t n32 = p.segs == 0 && segs == 64 ? split_frames(p.K, p.nframes, sms) : 0;
   if (n32 > 0) {
     const cudaError_t err = decode(0, n32, 32, pick(S32{}, std::false_type{}), lte_smem_bytes<32>(p.K));
     if (err != cudaSuccess) return err;

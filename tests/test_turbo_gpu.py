@@ -341,3 +341,32 @@ def test_tune_window(has_ref):
     bits = code.decode(llr)
     ref_bits, ref_app = checker.turbo_lte_decode(K, F.Approximate, 6, F.Serial, llr)
     assert_hard_parity(bits, ref_bits, msg, K, ref_app=ref_app)
+
+
+@pytest.mark.parametrize("K,frames,alg", [
+    (40, 1, 2), (40, 149, 1), (248, 3, 2), (256, 2, 2), (504, 5, 0), (512, 148, 2), (1024, 149, 2), (2112, 3, 1), (6144, 2, 2)])
+def test_windowed_staging_and_narrow_shapes(K, frames, alg):
+    """Frames the CTAs stage themselves (up to one per SM) and staged by a launch of their
+    own, on either side of the sizes where short frames take fewer threads: each segment
+    count decodes like the generic kernel, and a frame alone like the same frame in the
+    batch (decoded frames at 2 dB; all of a frame's segments are walked from its ends
+    where K <= 248, and the decisions are the same there in every frame)."""
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    code = F.Turbo.lte(K, F.Turbo.DecoderOptions().algorithm(alg).iterations(4))
+    msg = ch.random_bits(frames * K, K + frames)
+    llr = ch.awgn_llr(code.encode(msg), 2.0, K / code.paritySize(), K, np.float32)
+    got = code.decode(llr)
+    code.setKernel("generic")
+    ref = code.decode(llr)
+    code.setKernel("auto")
+    assert_hard_parity(got, ref, msg, K)
+    first = code.decode(llr[:code.paritySize()])
+    ok = frame_ok(ref, msg, K)
+    assert not ok[0] and K > 248 or np.array_equal(first, got[:K])
+    for segs in (32, 64, 128):
+        code.setWindowSegments(segs)
+        other = code.decode(llr)
+        assert_hard_parity(other, ref, msg, K)
+        if K <= 80:  # every segment is walked from the frame's ends
+            assert np.array_equal(other, got), segs
