@@ -192,7 +192,7 @@ ScratchPlan plan_scratch(fecl_codec_s* c, uint64_t n, bool lte_fast, bool soft) 
     sp.o2 = cv.take(n * P * 4);
     sp.o3 = cv.take(n * X * 4);
     sp.o4 = cv.take(n * X * 4);
-    sp.o5 = cv.take(n * uint64_t(c->tdev.max_steps) * c->tdev.max_states * 4);
+    sp.o5 = cv.take(fecl::turbo_generic_metrics_bytes(c->tdev, int64_t(n)));
   }
   sp.bytes = cv.off;
   return sp;

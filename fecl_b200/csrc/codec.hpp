@@ -302,6 +302,7 @@ struct fecl_codec_s {
     tdev.state = int32_t(turbo->state_size());
     tdev.tail = int32_t(turbo->syst_tail_size());
     tdev.max_steps = 0;
+    tdev.cta_ok = 1;
     tdev.max_states = 0;
     for (size_t j = 0; j < cs.size(); ++j) {
       const auto& c = cs[j];
@@ -321,6 +322,15 @@ struct fecl_codec_s {
       std::vector<uint32_t> padded_perm(c.perm);
       padded_perm.resize(c.perm.size() + 16, 0);
       upload_trellis(c.trellis, padded_perm, k);
+      std::vector<bool> seen(turbo->msg_size(), false);
+      for (uint32_t i : c.perm) {
+        if (i >= seen.size() || seen[i]) {
+          tdev.cta_ok = 0;
+          break;
+        }
+        seen[i] = true;
+      }
+      if (!k.pred || c.trellis.output_size > 6 || (k.input_count != 2 && k.input_count != 4)) tdev.cta_ok = 0;
       tdev.max_steps = std::max(tdev.max_steps, int32_t(c.length + c.tail));
       tdev.max_states = std::max(tdev.max_states, int32_t(c.trellis.state_count));
     }

@@ -45,6 +45,32 @@ inline LinearLut make_linear_lut() {
   return l;
 }
 
+// The same table as (slope, value) pairs of its intervals, with a last pair of zeros for
+// everything from 3.5 on; kernels that look it up copy it to shared memory.
+struct LinearPairs {
+  float2 v[8];
+};
+
+inline LinearPairs make_linear_pairs() {
+  const LinearLut l = make_linear_lut();
+  LinearPairs t;
+  for (int i = 0; i < 8; ++i) t.v[i] = i < 7 ? make_float2(l.y[i + 1] - l.y[i], l.y[i]) : make_float2(0.0f, 0.0f);
+  return t;
+}
+
+// LinearLogSum::sum (src/detail/LlrMetrics.h:107-112): max plus the table's value at |a - b|,
+// nothing where a == b.  The value is lut_log1pexpm's, without branches or conversions: floor(x)
+// for x in [0, 7] is the low bits of x + 2^23 rounded toward zero, and one 8-byte shared
+// load fetches the interval.  Lanes look up different entries, which constant memory serves
+// one address at a time.
+__device__ __forceinline__ float linear_sum(const float2* pairs, float a, float b) {
+  const float x = fminf(2.0f * fabsf(a - b), 7.0f);  // 7 also for two equal infinities
+  const float up = __fadd_rz(x, 8388608.0f);
+  const float2 e = pairs[__float_as_uint(up) & 7u];
+  const float r = fmaxf(a, b) + __fmaf_rn(e.x, x - (up - 8388608.0f), e.y);
+  return a == b ? a : r;
+}
+
 // Runs `upload` (which fills a translation unit's __constant__ tables) once per
 // device, with that device current.  __constant__ memory is per device, so a
 // process that decodes on several GPUs needs one upload on each.

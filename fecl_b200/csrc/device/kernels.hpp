@@ -199,6 +199,8 @@ struct TurboDeviceCode {
   TurboDeviceConstituent c[kMaxConstituents];
   const float* sf = nullptr;  // [n][iterations] resolved scaling
   int32_t algorithm = 1, iterations = 6, scheduling = 0;
+  // every constituent has a predecessor table and an interleaver of distinct indices: a CTA decodes a frame
+  int32_t cta_ok = 0;
   // Custom scheduling: stage s holds activations [stage_ptr[s], stage_ptr[s+1]);
   // activation a decodes constituent act_con[a] with a-priori input from the
   // constituents transfer[act_tptr[a] .. act_tptr[a+1]) (each list sorted).
@@ -229,9 +231,11 @@ struct TurboRun {
   float* parity_buf = nullptr;  // [nframes][parity]
   float* ext = nullptr;         // [nframes][state]
   float* ext_buf = nullptr;     // [nframes][state]
-  float* alpha = nullptr;       // [nframes][max_steps * max_states]
+  float* alpha = nullptr;       // turbo_generic_metrics_bytes
 };
 
+// Scratch for the trellis metrics (TurboRun::alpha).
+size_t turbo_generic_metrics_bytes(const TurboDeviceCode& code, int64_t nframes);
 cudaError_t launch_turbo_generic(const TurboDeviceCode& code, const TurboRun& run, cudaStream_t stream);
 
 // Windowed decoder for two constituents of the LTE RSC with Tail termination.

@@ -69,11 +69,6 @@ constexpr Tol kDecodeTol = {1e-3f, 1e-5f};
 constexpr Tol kSoftTol = {1e-6f, 1e-6f};
 constexpr int kDefaultSegs = 64;
 
-// The Linear table as (slope, value) pairs of its intervals, and a last pair of zeros for
-// everything from 3.5 on; copied to shared memory by the kernels that look it up.
-struct LinearPairs {
-  float2 v[8];
-};
 __constant__ LinearPairs c_lut;
 __shared__ float2 s_lut[8];
 
@@ -84,19 +79,9 @@ __shared__ float2 s_lut[8];
 __host__ __device__ constexpr int lte_next(int s, int u) { return (s >> 1) | (((u ^ s ^ (s >> 1)) & 1) << 2); }
 __host__ __device__ constexpr int lte_out(int s, int u) { return (u ^ (s >> 1) ^ (s >> 2)) & 1; }
 
-// The recursive log-sums (src/detail/LlrMetrics.h:88-121): max, or max plus the table's value
-// at |a - b| (nothing where a == b).  The lookup is lut_log1pexpm's, without branches or
-// conversions: floor(x) for x in [0, 7] is the low bits of x + 2^23 rounded toward zero,
-// and one 8-byte shared load fetches the interval.  Lanes look up different
-// entries, which constant memory serves one address at a time.
 template <int ALG>
 __device__ __forceinline__ float lsum(float a, float b) {
-  if (ALG == kApproximate) return fmaxf(a, b);
-  const float x = fminf(2.0f * fabsf(a - b), 7.0f);  // 7 also for two equal infinities
-  const float up = __fadd_rz(x, 8388608.0f);
-  const float2 e = s_lut[__float_as_uint(up) & 7u];
-  const float r = fmaxf(a, b) + __fmaf_rn(e.x, x - (up - 8388608.0f), e.y);
-  return a == b ? a : r;
+  return ALG == kApproximate ? fmaxf(a, b) : linear_sum(s_lut, a, b);
 }
 
 // max(a, b, c) in one instruction (the three-input form of max.f32, sm_100): the same
@@ -1265,9 +1250,7 @@ int64_t split_frames(int K, int64_t nframes, int sms) {
 cudaError_t turbo_lte_init() {
   static std::atomic<unsigned long long> done{0};
   return once_per_device(done, [] {
-    const LinearLut l = make_linear_lut();
-    LinearPairs t;
-    for (int i = 0; i < 8; ++i) t.v[i] = i < 7 ? make_float2(l.y[i + 1] - l.y[i], l.y[i]) : make_float2(0.0f, 0.0f);
+    const LinearPairs t = make_linear_pairs();
     return cudaMemcpyToSymbol(c_lut, &t, sizeof(t));
   });
 }
