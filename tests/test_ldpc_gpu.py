@@ -437,3 +437,30 @@ def test_persistent_launch_equals_launch_per_pass(alg, precision, frames, n):
     assert np.all(outs[1][1] > 0)
     for a, b in zip(outs[1], outs[-1]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,rate,frames", [(16200, (1, 2), 17), (16200, (3, 5), 64), (16200, (8, 9), 65), (64800, (1, 2), 40),
+                                           (64800, (9, 10), 130), ("gallager", None, 100)])
+def test_in_place_messages_equal_the_soft_path(n, rate, frames):
+    """FP16 hard decisions with the messages turned around in place (groups of 8 to 32
+    lanes, a partial last group, bits of every degree class, message sizes that are no
+    multiple of 4) against the decisions of the soft path, which keeps the
+    a-posteriori values: equal bits, and iteration counts of frames alone and in the batch."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    H = F.Ldpc.Gallager.matrix(2048, 3, 5, 0) if n == "gallager" else F.Ldpc.DvbS2.matrix(n, Fraction(*rate))
+    opts = F.Ldpc.DecoderOptions().algorithm(F.Approximate).iterations(25).scalingFactor(0.75).precision(1)
+    code = F.Ldpc(F.Ldpc.EncoderOptions(H), opts)
+    K, N = code.msgSize(), code.paritySize()
+    msg = ch.random_bits(frames * K, 90)
+    ebn0 = np.linspace(0.5, 5.0, frames)
+    llr = torch.from_numpy(ch.awgn_llr_per_frame(code.encode(msg), N, ebn0, K / N, 90, np.float32)).cuda()
+    bits, its = code.decode(llr, iterations=True)
+    out = code.soDecode(F.Codec.Input().parity(llr), F.Codec.Output(np.float32).msg())
+    assert torch.equal(bits, (out.msg() >= 0).to(torch.uint8))
+    for f in (0, frames // 2, frames - 1):  # a group of 2 lanes keeps the a-posteriori values too
+        one, it = code.decode(llr[f * N:(f + 1) * N], iterations=True)
+        assert torch.equal(one, bits[f * K:(f + 1) * K]) and int(it[0]) == int(its[f])
+    offset = torch.zeros(frames * K + 1, dtype=torch.uint8, device="cuda")
+    assert torch.equal(code.decode(llr, out=offset[1:]), bits)
