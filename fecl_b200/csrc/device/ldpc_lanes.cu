@@ -26,6 +26,17 @@
 //
 // Messages may be stored in FP16 or in saturated int8 (Q5.2, step 1/4, +-31.75);
 // every sum and every boxplus runs in FP32.
+//
+// FP32 messages keep no a-posteriori values: the bit pass (flow_bit) turns each message c of
+// the frames that go on into v = app - c in place, the check pass's own subtraction, and
+// leaves the signs of app as words of frame bits; the check pass (flow_check) then reads a
+// row's messages in order, without column indices or a gather, and takes the row's syndrome as
+// the xor of the sign words of its bits.  A retired frame's messages stay what its last
+// check pass left, which the soft outputs are sums of.  The values are the same bit for bit,
+// in a smaller working set (DVB-S2 normal r=9/10: 33 MB a group instead of 41).
+// DVB-S2 normal r=9/10 x 100, min-sum, <= 50 iterations: 4.69 ms against 6.94; short r=1/2 x 64,
+// Exact, 20 iterations, soft outputs: 0.580 ms against 0.591 (its check pass is bound by the
+// transform's arithmetic; a row per warp and 4 CTAs per SM, since two rows and 3 CTAs took 0.590).
 #include <cuda_fp16.h>
 #include <math.h>
 
@@ -231,6 +242,254 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) lanes_bit(LdpcLanesParams
   if (it >= 0 && blockIdx.x == 0 && threadIdx.x == 0) retire_group(p, it, g, active);
   if (!((active >> lane) & 1)) return;
   for (int b = int(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5); b < p.N; b += warps) bit_one<MSG>(p, g, b, lane);
+}
+
+// ---- FP32 messages in place ------------------------------------------------------------
+
+// The sign words of group g, in the place of its a-posteriori values: bit l of word b is set
+// where frame l's value at bit b is >= 0.
+__device__ __forceinline__ uint32_t* signs_of(const LdpcLanesParams& p, int g) {
+  return reinterpret_cast<uint32_t*>(p.app) + int64_t(g) * p.N;
+}
+
+// Rows per warp and step: two short rows in min-sum, for more loads in flight.
+template <int ALG, int DMAX>
+constexpr int flow_rows() { return DMAX <= 8 && ALG == kApproximate ? 2 : 1; }
+
+template <int ALG, int DMAX>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, ALG == kApproximate ? (DMAX > 16 ? 3 : 1) : (DMAX <= 8 ? 4 : 1)) flow_check(LdpcLanesParams p, int it, int g0) {
+  pdl_enter();
+  constexpr int kRows = flow_rows<ALG, DMAX>();
+  const int lane = lane_id();
+  const int warps = int(gridDim.x) * kWarpsPerBlock;
+  const bool check_syndrome = it > 0 && !p.fixed_iterations;
+  const float* sf_row = p.sf + size_t(it % p.n_sf) * p.sf_stride;
+  const int g = g0 + int(blockIdx.y);
+  const uint32_t active = active_of(p, it)[g];
+  if (active == 0) return;  // the same for the whole block (one group per grid row)
+  if constexpr (ALG == kLinear) share_lut();
+  const bool mine = (active >> lane) & 1;
+  const uint32_t* signs = signs_of(p, g);
+  const float* cg = static_cast<const float*>(p.c2v) + int64_t(g) * p.E * kLanes + lane;
+  uint32_t bad = 0;
+  const int w0 = int(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
+  for (int r = w0 * kRows; r < p.M; r += warps * kRows) {
+    float v[kRows][DMAX];
+    uint32_t e0[kRows];
+    int d[kRows];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      e0[q] = 0;
+      d[q] = 0;
+      if (r + q < p.M) {
+        e0[q] = __ldg(p.row_ptr + r + q);
+        d[q] = int(__ldg(p.row_ptr + r + q + 1) - e0[q]);
+      }
+      const float* row = cg + int64_t(e0[q]) * kLanes;
+#pragma unroll
+      for (int j = 0; j < DMAX; ++j)
+        if (j < d[q]) v[q][j] = row[j * kLanes];
+    }
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      if (check_syndrome)
+        bad |= __reduce_xor_sync(0xffffffffu, lane < d[q] ? signs[__ldg(p.col_idx + e0[q] + lane)] : 0u);
+      if (d[q] > 0) store_row<ALG, 0, DMAX>(p, g, e0[q], d[q], lane, sf_row, v[q], mine);
+    }
+  }
+  bad &= active;
+  if (bad && lane == 0) atomicOr(fail_of(p, it) + g, bad);
+}
+
+constexpr int kFlowBits = 2;  // neighbouring bits per warp and step, loaded together where their degrees agree
+
+// B neighbouring bits of D edges each: their a-posteriori values, their messages turned around
+// for the lanes that go on.  zero: every message is 0.
+template <int D, int B>
+__device__ __forceinline__ void flow_bits_d(float* cg, const uint32_t* edges, float (&acc)[B], bool zero, bool go_on) {
+  uint32_t e[B * D];
+  float x[B * D];
+#pragma unroll
+  for (int j = 0; j < B * D; ++j) e[j] = __ldg(edges + j);
+#pragma unroll
+  for (int j = 0; j < B * D; ++j) x[j] = zero ? 0.0f : cg[int64_t(e[j]) * kLanes];
+#pragma unroll
+  for (int i = 0; i < B; ++i)
+#pragma unroll
+    for (int j = 0; j < D; ++j) acc[i] += x[i * D + j];
+  if (go_on) {
+#pragma unroll
+    for (int j = 0; j < B * D; ++j) cg[int64_t(e[j]) * kLanes] = acc[j / D] - x[j];
+  }
+}
+
+// A bit of any degree, in runs of 8 edges (bit_one's order).
+__device__ __forceinline__ float flow_bit_any(float* cg, const uint32_t* edges, uint32_t deg, float acc, bool zero, bool go_on) {
+  constexpr uint32_t kRun = 8;
+  uint32_t e[kRun];
+  float x[kRun];
+  auto load = [&](uint32_t k) {
+#pragma unroll
+    for (uint32_t j = 0; j < kRun; ++j) e[j] = k + j < deg ? __ldg(edges + k + j) : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < kRun; ++j) x[j] = k + j < deg && !zero ? cg[int64_t(e[j]) * kLanes] : 0.0f;
+  };
+  for (uint32_t k = 0; k < deg; k += kRun) {
+    load(k);
+#pragma unroll
+    for (uint32_t j = 0; j < kRun; ++j)
+      if (k + j < deg) acc += x[j];
+  }
+  if (!go_on) return acc;
+  for (uint32_t k = 0; k < deg; k += kRun) {
+    if (deg > kRun) load(k);
+#pragma unroll
+    for (uint32_t j = 0; j < kRun; ++j)
+      if (k + j < deg) cg[int64_t(e[j]) * kLanes] = acc - x[j];
+  }
+  return acc;
+}
+
+// Bit pass after the check pass of iteration `it`, or with it < 0 the first one, over the
+// staged messages (zero: there are none).  Block (0, y) retires frames, as in lanes_bit.
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) flow_bit(LdpcLanesParams p, int it, int g0) {
+  pdl_enter();
+  const int lane = lane_id();
+  const int warps = int(gridDim.x) * kWarpsPerBlock;
+  const int g = g0 + int(blockIdx.y);
+  const bool first = it < 0, zero = first && !p.state_in;
+  const uint32_t active = active_of(p, first ? 0 : it)[g];
+  uint32_t on = active;
+  if (!first) {
+    if (it == p.iterations - 1) on = 0;
+    else if (it > 0 && !p.fixed_iterations) on &= fail_of(p, it)[g];
+    if (blockIdx.x == 0 && threadIdx.x == 0) retire_group(p, it, g, active);
+  }
+  if (active == 0) return;
+  const bool go_on = (on >> lane) & 1;
+  const bool whole = first || active == 0xffffffffu;  // no retired frame, whose sign stays
+  uint32_t* signs = signs_of(p, g);
+  float* cg = static_cast<float*>(p.c2v) + int64_t(g) * p.E * kLanes + lane;
+  const float* chan = p.chan + int64_t(g) * p.N * kLanes + lane;
+  for (int b0 = (int(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5)) * kFlowBits; b0 < p.N; b0 += warps * kFlowBits) {
+    const int n = min(kFlowBits, p.N - b0);
+    uint32_t k[kFlowBits + 1], old[kFlowBits];
+    float acc[kFlowBits];
+#pragma unroll
+    for (int i = 0; i <= kFlowBits; ++i) k[i] = __ldg(p.col_ptr + b0 + min(i, n));
+#pragma unroll
+    for (int i = 0; i < kFlowBits; ++i) {
+      acc[i] = i < n ? chan[int64_t(b0 + i) * kLanes] : 0.0f;
+      old[i] = !whole && lane == 0 && i < n ? signs[b0 + i] : 0u;
+    }
+    const uint32_t deg = k[1] - k[0];
+    bool same = n == kFlowBits;
+#pragma unroll
+    for (int i = 1; i < kFlowBits; ++i) same = same && k[i + 1] - k[i] == deg;
+    const uint32_t* edges = p.col_edges + k[0];
+    switch (same ? deg : 0u) {
+      case 1: flow_bits_d<1, kFlowBits>(cg, edges, acc, zero, go_on); break;
+      case 2: flow_bits_d<2, kFlowBits>(cg, edges, acc, zero, go_on); break;
+      case 3: flow_bits_d<3, kFlowBits>(cg, edges, acc, zero, go_on); break;
+      case 4: flow_bits_d<4, kFlowBits>(cg, edges, acc, zero, go_on); break;
+      default:
+#pragma unroll
+        for (int i = 0; i < kFlowBits; ++i)
+          acc[i] = flow_bit_any(cg, p.col_edges + k[i], k[i + 1] - k[i], acc[i], zero, go_on);
+    }
+    const uint32_t mask = first ? 0xffffffffu : active;
+#pragma unroll
+    for (int i = 0; i < kFlowBits; ++i) {
+      const uint32_t w = __ballot_sync(0xffffffffu, acc[i] >= 0.0f);
+      if (i < n && lane == 0) signs[b0 + i] = (old[i] & ~mask) | (w & mask);
+    }
+  }
+}
+
+// Staging for the in-place passes: a tile of 32 bits of a group's 32 frames goes through
+// shared memory, so that the frame-major reads and the lane-minor writes are both contiguous.
+// The messages (state_in) are staged by lanes_stage's loop.  Block (0, y) writes the masks.
+__global__ void __launch_bounds__(256) flow_stage(LdpcLanesParams p) {
+  __shared__ float tile[kLanes][33];
+  const int g = int(blockIdx.y), lane = lane_id(), warp = threadIdx.x >> 5, b0 = int(blockIdx.x) * 32;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int frame = q * 8 + warp, b = b0 + lane;
+    const int64_t f = int64_t(g) * kLanes + frame;
+    float x = 0.0f;
+    if (f < p.nframes && b < p.N) {
+      x = load_llr(p.llr, p.llr_dtype, f * p.N + b);
+      if (p.syst_in && b < p.msg) x += load_llr(p.syst_in, p.llr_dtype, f * p.msg + b);
+    }
+    tile[frame][lane] = x;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int bit = q * 8 + warp;
+    if (b0 + bit < p.N) p.chan[(int64_t(g) * p.N + b0 + bit) * kLanes + lane] = tile[lane][bit];
+  }
+  if (p.state_in) {
+    float* c2v = static_cast<float*>(p.c2v) + int64_t(g) * p.E * kLanes;
+    for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < p.E * kLanes; i += int64_t(gridDim.x) * 256) {
+      const int64_t f = int64_t(g) * kLanes + i % kLanes;
+      c2v[i] = f < p.nframes ? load_llr(p.state_in, p.llr_dtype, f * p.E + i / kLanes) : 0.0f;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int64_t left = p.nframes - int64_t(g) * kLanes;
+    p.active[g] = left >= kLanes ? 0xffffffffu : ((1u << left) - 1u);
+    p.active[p.groups + g] = 0;
+    p.fail[g] = 0;
+    p.fail[p.groups + g] = 0;
+  }
+}
+
+// Outputs of a tile of 32 bits of group blockIdx.y: decisions from the sign words, extrinsic
+// values as sums of the messages in edge order, through shared memory to frame-major stores.
+__global__ void __launch_bounds__(256) flow_finish(LdpcLanesParams p) {
+  __shared__ float ext[kLanes][33], post[kLanes][33];
+  const int g = int(blockIdx.y), lane = lane_id(), warp = threadIdx.x >> 5, b0 = int(blockIdx.x) * 32;
+  const bool soft = p.msg_out || p.syst_out || p.parity_out;
+  if (soft) {
+    const float* cg = static_cast<const float*>(p.c2v) + int64_t(g) * p.E * kLanes + lane;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int bit = q * 8 + warp, b = b0 + bit;
+      if (b >= p.N) continue;
+      float x = 0.0f;
+      for (uint32_t k = __ldg(p.col_ptr + b); k < __ldg(p.col_ptr + b + 1); ++k)
+        x += cg[int64_t(__ldg(p.col_edges + k)) * kLanes];
+      ext[lane][bit] = x;
+      post[lane][bit] = p.chan[(int64_t(g) * p.N + b) * kLanes + lane] + x;
+    }
+    __syncthreads();
+  }
+  const int b = b0 + lane;
+  const uint32_t word = p.hard && b < p.msg ? signs_of(p, g)[b] : 0u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int frame = q * 8 + warp;
+    const int64_t f = int64_t(g) * kLanes + frame;
+    if (f >= p.nframes || b >= p.N) continue;
+    if (p.hard && b < p.msg) p.hard[f * p.msg + b] = uint8_t((word >> frame) & 1u);
+    if (p.parity_out) store_llr(p.parity_out, p.out_dtype, f * p.N + b, ext[frame][lane]);
+    if (b < p.msg) {
+      if (p.syst_out) store_llr(p.syst_out, p.out_dtype, f * p.msg + b, ext[frame][lane]);
+      if (p.msg_out) store_llr(p.msg_out, p.out_dtype, f * p.msg + b, post[frame][lane]);
+    }
+  }
+  if (p.state_out) {
+    const float* cg = static_cast<const float*>(p.c2v) + int64_t(g) * p.E * kLanes;
+    for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < p.E * kLanes; i += int64_t(gridDim.x) * 256) {
+      const int64_t f = int64_t(g) * kLanes + i % kLanes;
+      if (f < p.nframes) store_llr(p.state_out, p.out_dtype, f * p.E + i / kLanes, cg[i]);
+    }
+  }
+  if (p.iters && blockIdx.x == 0 && threadIdx.x < kLanes) {
+    const int64_t f = int64_t(g) * kLanes + threadIdx.x;
+    if (f < p.nframes) p.iters[f] = p.iters_ws[f];
+  }
 }
 
 // Persistent decoder for a small batch (at most kPersistGroups groups, all in one wave):
@@ -467,9 +726,33 @@ cudaError_t launch_persistent(LdpcLanesParams p, cudaStream_t s) {
   return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarpsPerBlock * 32, args);
 }
 
+// A decode with FP32 messages in place; waves as below, of the smaller working set.
+template <int ALG, int DMAX>
+cudaError_t run_flow(const LdpcLanesParams& p, cudaStream_t s) {
+  const int wave = wave_for(p, int64_t(kLanes) * 4 * (int64_t(p.N) + p.E) + 4 * int64_t(p.N));
+  const dim3 tiles(unsigned((p.N + 31) / 32), unsigned(p.groups));
+  flow_stage<<<tiles, 256, 0, s>>>(p);
+  for (int w0 = 0; w0 < p.groups; w0 += wave) {
+    const int nw = p.groups - w0 < wave ? p.groups - w0 : wave;
+    const dim3 gbit = grid_for((p.N + kFlowBits - 1) / kFlowBits, nw);
+    constexpr int kRows = flow_rows<ALG, DMAX>();
+    const dim3 gchk = grid_for((p.M + kRows - 1) / kRows, nw);
+    cudaError_t e = launch_pdl(flow_bit, gbit, dim3(kWarpsPerBlock * 32), s, p, -1, w0);
+    for (int it = 0; e == cudaSuccess && it < p.iterations; ++it) {
+      e = launch_pdl(flow_check<ALG, DMAX>, gchk, dim3(kWarpsPerBlock * 32), s, p, it, w0);
+      if (e == cudaSuccess) e = launch_pdl(flow_bit, gbit, dim3(kWarpsPerBlock * 32), s, p, it, w0);
+    }
+    if (e != cudaSuccess) return e;
+  }
+  flow_finish<<<tiles, 256, 0, s>>>(p);
+  return cudaGetLastError();
+}
+
 template <int ALG, int MSG, int DMAX>
 cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   if (p.groups > 65535) return cudaErrorInvalidValue;
+  if constexpr (MSG == 0)
+    if (p.persist <= 0) return run_flow<ALG, DMAX>(p, s);
   const int wave = wave_for(p, group_bytes(p));
   const dim3 gs((148 * 8 + p.groups - 1) / p.groups, p.groups);
   lanes_stage<MSG><<<gs, 256, 0, s>>>(p);

@@ -464,3 +464,38 @@ def test_in_place_messages_equal_the_soft_path(n, rate, frames):
         assert torch.equal(one, bits[f * K:(f + 1) * K]) and int(it[0]) == int(its[f])
     offset = torch.zeros(frames * K + 1, dtype=torch.uint8, device="cuda")
     assert torch.equal(code.decode(llr, out=offset[1:]), bits)
+
+
+@pytest.mark.parametrize("alg,n,rate,frames", [(0, 16200, (1, 2), 33), (1, 16200, (4, 5), 31), (2, 16200, (8, 9), 65),
+                                               (2, 64800, (3, 5), 40), (2, "gallager", None, 70)])
+def test_in_place_fp32_messages_equal_the_persistent_launch(alg, n, rate, frames):
+    """FP32 messages turned around in place against the persistent launch, which keeps the
+    a-posteriori values: bits, iteration counts and every soft output equal, with frames
+    that retire at different iterations, a-priori and state inputs, and a partial last group."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    H = F.Ldpc.Gallager.matrix(2048, 3, 5, 0) if n == "gallager" else F.Ldpc.DvbS2.matrix(n, Fraction(*rate))
+    opts = F.Ldpc.DecoderOptions().algorithm(alg).iterations(12).scalingFactor(0.75 if alg == 2 else 1.0)
+    code = F.Ldpc(F.Ldpc.EncoderOptions(H), opts)
+    K, N, E = code.msgSize(), code.paritySize(), code.stateSize()
+    msg = ch.random_bits(frames * K, 91)
+    llr = torch.from_numpy(ch.awgn_llr_per_frame(code.encode(msg), N, np.linspace(0.5, 6.0, frames), K / N, 91,
+                                                 np.float32)).cuda()
+    g = torch.Generator(device="cuda").manual_seed(91)
+    syst = 0.2 * torch.randn(frames * K, device="cuda", generator=g)
+    state = 0.2 * torch.randn(frames * E, device="cuda", generator=g)
+
+    def everything():
+        bits, its = code.decode(llr, iterations=True)
+        got = [bits, its]
+        for inp in (F.Codec.Input().parity(llr), F.Codec.Input().parity(llr).syst(syst).state(state)):
+            out = code.soDecode(inp, F.Codec.Output(np.float32).msg().syst().parity().state())
+            got += [out.msg(), out.syst(), out.parity(), out.state()]
+        return got
+
+    code.setPersistent(0)
+    mine = everything()
+    code.setPersistent(1)
+    for a, b in zip(mine, everything()):
+        assert torch.equal(a, b)
