@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "kernels.hpp"
+#include "trellis_encode.cuh"
 
 namespace fecl {
 namespace {
@@ -298,6 +299,15 @@ __global__ void __launch_bounds__(32) viterbi_warp(TurboDeviceConstituent k, Vit
   } while (__any_sync(0xffffffffu, again));
 }
 
+__global__ void __launch_bounds__(kEncodeThreads) conv_encode_cta(const __grid_constant__ TurboDeviceConstituent c,
+                                                                  const uint8_t* msg, uint8_t* parity) {
+  __shared__ EncodeShared sh;
+  extern __shared__ __align__(16) uint8_t s[];
+  const int64_t f = blockIdx.x;
+  encode_constituent(c, msg + f * c.msg_size, nullptr, parity + f * c.parity_size, nullptr, sh, s);
+}
+
+// A thread per frame, for trellises and lengths beyond conv_encode_cta's.
 __global__ void conv_encode_kernel(TurboDeviceConstituent c, const uint8_t* msg, uint8_t* parity, int64_t nframes) {
   const int64_t f = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (f >= nframes) return;
@@ -377,6 +387,12 @@ cudaError_t launch_viterbi(const TurboDeviceConstituent& k, const ViterbiRun& r,
 cudaError_t launch_conv_encode(const TurboDeviceConstituent& c, const uint8_t* msg, uint8_t* parity, int64_t nframes,
                                cudaStream_t s) {
   if (nframes <= 0) return cudaSuccess;
+  if (encode_by_cta(c) && nframes <= 0x7fffffff) {
+    const cudaError_t e = cudaFuncSetAttribute(conv_encode_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, c.length);
+    if (e != cudaSuccess) return e;
+    conv_encode_cta<<<unsigned(nframes), kEncodeThreads, size_t(c.length), s>>>(c, msg, parity);
+    return cudaGetLastError();
+  }
   conv_encode_kernel<<<unsigned((nframes + 63) / 64), 64, 0, s>>>(c, msg, parity, nframes);
   return cudaGetLastError();
 }

@@ -111,3 +111,23 @@ def test_ldpc_encoder_frames_per_cta_and_alignment(code, frames):
         buf = torch.zeros(offset + msg.size, dtype=torch.uint8, device="cuda")
         buf[offset:] = torch.from_numpy(msg).cuda() | 0xFE if offset == 1 else torch.from_numpy(msg).cuda()
         assert torch.equal(c.encode(buf[offset:]), want), offset
+
+
+@pytest.mark.parametrize("K,frames", [(1, 2), (40, 300), (127, 3), (128, 2), (129, 2), (6144, 5)])
+def test_trellis_encoders_by_chunks(K, frames):
+    """One step, chunks of one step (threads without any), a chunk more than the threads;
+    4 to 64 states, one and two inputs, one to three outputs.  Bits: equal to the host's."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    specs = [([4], [[0o15]], [0o13]), ([7], [[0o171, 0o133]], None), ([3, 3], [[0o5, 0o3, 0], [0, 0o3, 0o7]], [0o7, 0o5])]
+    codes = []
+    for spec in specs:
+        for term in (0, 1):
+            codes.append(F.Convolutional(F.Convolutional.EncoderOptions(F.Trellis(*spec), K).termination(term)))
+    perms = [np.arange(K, dtype=np.uint32), np.random.default_rng(K).permutation(K).astype(np.uint32)]
+    codes.append(F.Turbo(F.Turbo.EncoderOptions([F.Trellis(*T17)], perms), F.Turbo.DecoderOptions()))
+    for i, code in enumerate(codes):
+        msg = ch.random_bits(frames * code.msgSize(), 63 + i)
+        want = code.encode(msg)
+        assert np.array_equal(want, code.encode(torch.from_numpy(msg).cuda()).cpu().numpy()), i
