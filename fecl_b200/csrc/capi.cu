@@ -205,6 +205,7 @@ fecl::LdpcLanesParams lanes_params(fecl_codec_s* c, const Launch& d, uint64_t n,
   r.N = L.N;
   r.msg = L.msg;
   r.d_max = L.d_max;
+  r.c_max = L.c_max;
   r.E = L.E;
   r.row_ptr = L.row_ptr;
   r.col_idx = L.col_idx;
@@ -219,6 +220,7 @@ fecl::LdpcLanesParams lanes_params(fecl_codec_s* c, const Launch& d, uint64_t n,
   r.msg_type = c->ldpc->decoder().precision;
   r.wave_groups = c->lanes_wave;
   r.persist = c->lanes_persist;
+  r.alone = d.alone;
   r.nframes = int64_t(n);
   r.llr = d.llr;
   r.llr_dtype = in_dtype;
@@ -441,6 +443,7 @@ void run_decode(fecl_codec_s* c, const fecl_so_io* io, uint64_t n, uint8_t* hard
     d.parity_out = io->parity_out;
     d.state_out = io->state_out;
     d.scratch = c->ws.as<char>();
+    d.alone = true;
     launch_decode(c, d, sp, n, io->in_dtype, io->out_dtype, soft, lte_fast, user_stream);
     c->mark(user_stream);
     return;
@@ -515,6 +518,7 @@ void run_decode(fecl_codec_s* c, const fecl_so_io* io, uint64_t n, uint8_t* hard
     if (io->parity_out) d.parity_out = base + o_po;
     if (io->state_out) d.state_out = base + o_sto;
     d.scratch = base + o_scr;
+    d.alone = nchunks == 1;
     launch_decode(c, d, sp, nk, io->in_dtype, io->out_dtype, soft, lte_fast, st);
     if (hard) cuda_check(cudaMemcpyAsync(hard + f0 * M, d.hard, nk * M, cudaMemcpyDeviceToHost, st), "copy out");
     if (iters) cuda_check(cudaMemcpyAsync(iters + f0, d.iters, nk * 4, cudaMemcpyDeviceToHost, st), "copy out");

@@ -183,6 +183,7 @@ struct fecl_codec_s {
     // per-bit edge lists in increasing edge order
     std::vector<uint32_t> cp(H.cols + 1, 0), ce(H.nnz());
     for (auto c : H.col_idx) cp[c + 1]++;
+    ldev.c_max = int32_t(*std::max_element(cp.begin(), cp.end()));
     for (uint32_t b = 0; b < H.cols; ++b) cp[b + 1] += cp[b];
     std::vector<uint32_t> fill(cp.begin(), cp.end() - 1);
     for (uint64_t e = 0; e < H.nnz(); ++e) ce[fill[H.col_idx[e]]++] = uint32_t(e);
@@ -532,6 +533,7 @@ struct Launch {
   int32_t* iters = nullptr;
   void *msg = nullptr, *syst_out = nullptr, *parity_out = nullptr, *state_out = nullptr;
   char* scratch = nullptr;
+  bool alone = false;  // the call's only decode on the device
 };
 
 // Scratch of the decoder kernels for n frames, with the offsets of its parts.

@@ -32,23 +32,23 @@ __device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned* error,
   __syncthreads();
   epoch += gridDim.x;
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(counter, 1u);
+    // the block's writes, ordered before this thread by the barrier above, are released with the arrival
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
     const unsigned long long t0 = global_ns();
     int good = 1;
-    while (load_acquire(counter) < epoch) {
+    // the failure flag and the clock are looked at once in 64 polls: a poll costs its load alone
+    for (unsigned polls = 1; load_acquire(counter) < epoch; ++polls) {
+      if (polls % 64 != 0) continue;
       if (load_acquire(error) != 0u) {
         good = 0;
         break;
       }
-      __nanosleep(64);
       if (global_ns() - t0 > kBarrierNs) {
         atomicExch(error, 1u);
         good = 0;
         break;
       }
     }
-    __threadfence();
     ok = good;
   }
   __syncthreads();

@@ -12,7 +12,7 @@ namespace fecl {
 // A check matrix laid out for the device: CSR by check (the edge order of the
 // soft state), plus for every bit the ids of its edges in increasing order.
 struct LdpcDeviceCode {
-  int32_t M = 0, N = 0, msg = 0, d_max = 0;
+  int32_t M = 0, N = 0, msg = 0, d_max = 0, c_max = 0;
   int64_t E = 0;
   const uint32_t* row_ptr = nullptr;    // [M+1]
   const uint32_t* col_idx = nullptr;    // [E]
@@ -49,7 +49,7 @@ cudaError_t launch_ldpc_flood(const LdpcDeviceCode& code, const LdpcRun& run, cu
 // Batched decoder with 32 frames per warp (one per lane), lane-minor scratch.
 struct LdpcLanesParams {
   // code
-  int32_t M = 0, N = 0, msg = 0, d_max = 0;
+  int32_t M = 0, N = 0, msg = 0, d_max = 0, c_max = 0;  // d_max, c_max: largest check and bit degree
   int64_t E = 0;
   const uint32_t* row_ptr = nullptr;
   const uint32_t* col_idx = nullptr;
@@ -60,7 +60,9 @@ struct LdpcLanesParams {
   int32_t algorithm = 2, iterations = 1, fixed_iterations = 0;
   int32_t msg_type = 0;  // 0 FP32, 1 FP16, 2 saturated int8 (Q5.2)
   int32_t wave_groups = 0;  // groups decoded together (0: as many as fit in 64 MiB of L2)
-  int32_t persist = 0;      // one persistent launch for small batches: 1 wherever it applies, 0 / -1 never
+  // one persistent launch for small batches: 1 wherever it applies, -1 never, 0 where it is the
+  // faster and the call is `alone`: not one of several decodes launched to run beside one another
+  int32_t persist = 0, alone = 0;
   // batch, frame-major caller buffers
   int64_t nframes = 0;
   const void* llr = nullptr;
@@ -88,7 +90,7 @@ struct LdpcLanesParams {
 size_t ldpc_lanes_scratch_bytes(int64_t N, int64_t E, int64_t nframes, int msg_type);
 // Cooperative launch of a persistent LDPC kernel, ordered after the previous one on
 // this device (ldpc_lanes.cu).
-cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, void** args);
+cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, size_t smem, void** args);
 cudaError_t launch_ldpc_lanes(LdpcLanesParams p, void* scratch, cudaStream_t stream);
 
 // Normalised min-sum with FP16 messages and packed half2 check-node arithmetic, two

@@ -692,7 +692,7 @@ std::mutex g_persist_mu;
 cudaEvent_t g_persist_ev[64] = {};
 }  // namespace
 
-cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, void** args) {
+cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, size_t smem, void** args) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -701,7 +701,7 @@ cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned block
   if (!g_persist_ev[dev] && (e = cudaEventCreateWithFlags(&g_persist_ev[dev], cudaEventDisableTiming)) != cudaSuccess)
     return e;
   if ((e = cudaStreamWaitEvent(s, g_persist_ev[dev], 0)) != cudaSuccess) return e;
-  if ((e = cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, 0, s)) != cudaSuccess) return e;
+  if ((e = cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, smem, s)) != cudaSuccess) return e;
   return cudaEventRecord(g_persist_ev[dev], s);
 }
 
@@ -723,7 +723,7 @@ cudaError_t launch_persistent(LdpcLanesParams p, cudaStream_t s) {
   if (blocks < 1) return cudaErrorInvalidConfiguration;
   if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
   void* args[] = {&p};
-  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarpsPerBlock * 32, args);
+  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarpsPerBlock * 32, 0, args);
 }
 
 // A decode with FP32 messages in place; waves as below, of the smaller working set.

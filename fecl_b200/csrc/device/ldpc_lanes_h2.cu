@@ -600,6 +600,136 @@ __global__ void __launch_bounds__(kWarps * 32) h2_persist(LdpcLanesParams p) {
     for (int i = threadIdx.x; i < ng * 64; i += blockDim.x) p.iters_ws[i] = -1;
 }
 
+// h2_persist for one narrow group (at most 16 frames).  Its passes are a few microseconds each
+// and a launch per pass is bound by the launches, those after the last frame has
+// retired included; here a pass costs a grid barrier and the kernel ends with the last
+// frame.  A warp works on the same rows and bits in every pass, so their index lists stay in
+// shared memory, a task's lists side by side over its slots, and a pass waits for one
+// load from L2 instead of three.  `rows` and `bits`: tasks (32 / W rows or bits) per warp.
+// One DVB-S2 short r=2/3 frame in the waterfall: 168 us a call against 232 (persists_alone has more).
+constexpr int kNarrowThreads = 512;
+
+__host__ __device__ inline size_t narrow_words_per_warp(int d_max, int c_max, int W, int rows, int bits) {
+  return size_t(32 / W) * (size_t(rows) * (2 + d_max) + size_t(bits) * (1 + c_max));
+}
+
+template <int DMAX, int W>
+__global__ void __launch_bounds__(kNarrowThreads) h2_persist_narrow(LdpcLanesParams p, int rows, int bits) {
+  constexpr int kSlots = 32 / W, kRun = 8;
+  extern __shared__ uint32_t lists[];
+  const int lane = threadIdx.x & 31, sub = lane % W, slot = lane / W;
+  const int warp = int(blockIdx.x) * (kNarrowThreads / 32) + (threadIdx.x >> 5);
+  const int warps = int(gridDim.x) * (kNarrowThreads / 32);
+  const int rstep = (2 + p.d_max) * kSlots, bstep = (1 + p.c_max) * kSlots;
+  uint32_t* rl = lists + (threadIdx.x >> 5) * (rows * rstep + bits * bstep) + slot;  // e0, degree, columns
+  uint32_t* bl = rl + rows * rstep;                                                  // degree, edges
+  for (int k = 0; k < rows; ++k) {
+    const int r = (warp + k * warps) * kSlots + slot;
+    const uint32_t e0 = r < p.M ? p.row_ptr[r] : 0u, d = r < p.M ? p.row_ptr[r + 1] - e0 : 0u;
+    uint32_t* q = rl + k * rstep;
+    if (sub == 0) q[0] = e0;
+    if (sub == 0) q[kSlots] = d;
+    for (uint32_t i = sub; i < d; i += W) q[(2 + i) * kSlots] = p.col_idx[e0 + i];
+  }
+  for (int k = 0; k < bits; ++k) {
+    const int b = (warp + k * warps) * kSlots + slot;
+    const uint32_t e0 = b < p.N ? p.col_ptr[b] : 0u, d = b < p.N ? p.col_ptr[b + 1] - e0 : 0u;
+    uint32_t* q = bl + k * bstep;
+    if (sub == 0) q[0] = d;
+    for (uint32_t i = sub; i < d; i += W) q[(1 + i) * kSlots] = p.col_edges[e0 + i];
+  }
+  __syncwarp();
+
+  __half2* cg = static_cast<__half2*>(p.c2v) + sub;
+  float2* app = reinterpret_cast<float2*>(p.app) + sub;
+  const float2* chan = reinterpret_cast<const float2*>(p.chan) + sub;
+  const bool keep_all = p.msg_out || p.syst_out || p.parity_out || p.state_out;
+  // bit_one over this warp's bits
+  auto bit_pass = [&](bool mx, bool my) {
+    for (int k = 0; k < bits; ++k) {
+      const int64_t at = int64_t((warp + k * warps) * kSlots + slot) * W;
+      if ((warp + k * warps) * kSlots + slot >= p.N) continue;
+      const uint32_t* q = bl + k * bstep;
+      const int deg = int(q[0]);
+      float2 acc = chan[at];
+      for (int i0 = 0; i0 < deg; i0 += kRun) {
+        __half2 x[kRun];
+#pragma unroll
+        for (int i = 0; i < kRun; ++i) x[i] = i0 + i < deg ? cg[int64_t(q[(1 + i0 + i) * kSlots]) * W] : __half2{};
+#pragma unroll
+        for (int i = 0; i < kRun; ++i)
+          if (i0 + i < deg) acc = __fadd2_rn(acc, __half22float2(x[i]));
+      }
+      if (mx && my) {
+        app[at] = acc;
+      } else {
+        float2 out = app[at];
+        if (mx) out.x = acc.x;
+        if (my) out.y = acc.y;
+        app[at] = out;
+      }
+    }
+  };
+  unsigned epoch = 0;
+  bit_pass(true, true);
+  // every thread follows the masks: those of the next iteration come from these and the failures
+  uint32_t ax = active_of(p, 0)[0], ay = active_of(p, 0)[1];
+  bool ok = grid_barrier(p.barrier, p.barrier + 1, epoch);
+  for (int it = 0; ok && it < p.iterations; ++it) {
+    const bool check_syndrome = it > 0 && !p.fixed_iterations;
+    const bool mx = (ax >> sub) & 1, my = (ay >> sub) & 1;
+    const float* sf = p.sf + size_t(it % p.n_sf) * p.sf_stride;
+    uint32_t bx = 0, by = 0;
+    // check_rows over this warp's rows
+    for (int k = 0; k < rows; ++k) {
+      const uint32_t* q = rl + k * rstep;
+      Row<DMAX> w;
+      w.e0 = q[0];
+      w.d = int(q[kSlots]);
+      w.px = w.py = 0;
+      const float s = sf[w.d >= 2 ? w.d - 2 : 0];
+      const __half2* row = cg + int64_t(w.e0) * W;
+      float2 a[DMAX];
+#pragma unroll
+      for (int i = 0; i < DMAX; ++i)
+        if (i < w.d) {
+          a[i] = app[int64_t(q[(2 + i) * kSlots]) * W];
+          w.v[i] = row[i * W];
+        }
+#pragma unroll
+      for (int i = 0; i < DMAX; ++i) {
+        if (i < w.d) {
+          w.px ^= unsigned(a[i].x >= 0.0f);
+          w.py ^= unsigned(a[i].y >= 0.0f);
+          w.v[i] = half2_satfinite(__ffma2_rn(__half22float2(w.v[i]), make_float2(-1.0f, -1.0f), a[i]));
+        }
+      }
+      if (check_syndrome) {
+        bx |= fold_lanes<W>(__ballot_sync(0xffffffffu, w.d > 0 && w.px != 0));
+        by |= fold_lanes<W>(__ballot_sync(0xffffffffu, w.d > 0 && w.py != 0));
+      }
+      if (w.d > 0) store_row<DMAX, W>(p, 0, sub, w, __float2half2_rn(s), mx, my, keep_all);
+    }
+    if (lane == 0 && (bx & ax)) atomicOr(fail_of(p, it), bx & ax);
+    if (lane == 0 && (by & ay)) atomicOr(fail_of(p, it) + 1, by & ay);
+    if (!(ok = grid_barrier(p.barrier, p.barrier + 1, epoch))) break;
+    uint32_t on_x = ax, on_y = ay;
+    if (it == p.iterations - 1) on_x = on_y = 0;
+    else if (check_syndrome) {
+      on_x &= fail_of(p, it)[0];
+      on_y &= fail_of(p, it)[1];
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 2) retire_half<W>(p, it, 0, threadIdx.x);
+    if (mx || my) bit_pass(mx, my);
+    ax = on_x;
+    ay = on_y;
+    if ((ax | ay) == 0) break;
+    if (!(ok = grid_barrier(p.barrier, p.barrier + 1, epoch))) break;
+  }
+  if (!ok && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < 2 * W; i += blockDim.x) p.iters_ws[i] = -1;
+}
+
 // ---- several codes in one launch ------------------------------------------------
 
 // The groups of every job of a mixed batch (each job one code, its own scratch) whose
@@ -934,8 +1064,21 @@ __global__ void __launch_bounds__(kWarps * 32) h2_bit_many(LdpcMultiParams m, in
 // kPersistGroups groups, all in one wave, on a stream that is not capturing (the
 // per-pass launches are the built-in choice: see ldpc_lanes.cu).
 
-bool use_persistent(const LdpcLanesParams& p, int64_t wave, cudaStream_t s) {
-  if (p.persist <= 0 || p.groups > kPersistGroups || wave < p.groups) return false;
+// One narrow group of a code of at most kPersistBits bits takes the persistent launch by itself
+// when its call is the only decode under way: 1 to 16 DVB-S2 short frames, 50 iterations allowed,
+// took 80 to 105 us against 230 a dB above the waterfall (8 iterations), 175 to 220 against
+// 250 to 305 in it (18), and as long with frames that never converge (437 to 481 against 433 to
+// 535).  Frames of 64800 bits gained as much when they converged early but ran 8 to 20 %
+// longer when they did not, so they keep a launch per pass.  Groups of 2 lanes are widened
+// to 4, which touch whole sectors of app (457 us against 438).
+constexpr int kPersistBits = 20000;
+
+bool persists_alone(const LdpcLanesParams& p) {
+  return p.alone && p.persist == 0 && p.nframes <= 16 && p.N <= kPersistBits;
+}
+
+bool use_persistent(const LdpcLanesParams& p, int64_t wave, bool narrow, cudaStream_t s) {
+  if ((p.persist <= 0 && !narrow) || p.groups > kPersistGroups || wave < p.groups) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -960,7 +1103,29 @@ cudaError_t launch_persistent(LdpcLanesParams p, cudaStream_t s) {
   if (blocks < 1) return cudaErrorInvalidConfiguration;
   if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
   void* args[] = {&p};
-  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarps * 32, args);
+  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarps * 32, 0, args);
+}
+
+// One block per SM at most; cudaErrorInvalidConfiguration where the index lists do not fit.
+template <int DMAX, int W>
+cudaError_t launch_narrow(LdpcLanesParams p, cudaStream_t s) {
+  constexpr int kSlots = 32 / W, kBlockWarps = kNarrowThreads / 32;
+  int dev = 0, sms = 0, limit = 0;
+  cudaError_t e;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  const int row_tasks = (p.M + kSlots - 1) / kSlots, bit_tasks = (p.N + kSlots - 1) / kSlots;
+  const int need = ((row_tasks > bit_tasks ? row_tasks : bit_tasks) + kBlockWarps - 1) / kBlockWarps;
+  const int blocks = need < sms ? need : sms, warps = blocks * kBlockWarps;
+  int rows = (row_tasks + warps - 1) / warps, bits = (bit_tasks + warps - 1) / warps;
+  const size_t smem = kBlockWarps * narrow_words_per_warp(p.d_max, p.c_max, W, rows, bits) * 4;
+  if (blocks < 1 || smem + 1024 > size_t(limit)) return cudaErrorInvalidConfiguration;
+  auto kern = h2_persist_narrow<DMAX, W>;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
+  void* args[] = {&p, &rows, &bits};
+  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kNarrowThreads, smem, args);
 }
 
 // The grid of the staging and finishing kernels: 256 threads per block over the
@@ -1011,7 +1176,7 @@ cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   // scattered stores cost more than the gathers they save (one DVB-S2 short frame: 0.33 ms
   // against 0.25).
   if constexpr (W >= 8)
-    if (p.hard && !p.msg_out && !p.syst_out && !p.parity_out && !p.state_out && !p.syst_in && p.persist <= 0)
+    if (!persists_alone(p) && p.hard && !p.msg_out && !p.syst_out && !p.parity_out && !p.state_out && !p.syst_in && p.persist <= 0)
       return run_flow<DMAX, W>(p, s);
   constexpr int kSlots = 32 / W;
   const int64_t gb = int64_t(W) * (2 * 8 * int64_t(p.N) + 4 * p.E);
@@ -1021,8 +1186,11 @@ cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   const dim3 gs = stage_grid(p, W);
   h2_stage<W><<<gs, 256, 0, s>>>(p);
   bool done = false;
-  if (W == kLanes && use_persistent(p, wave, s)) {
-    const cudaError_t e = launch_persistent<DMAX>(p, s);
+  const bool narrow = W < kLanes && p.groups == 1 && persists_alone(p);
+  if ((W == kLanes || p.groups == 1) && use_persistent(p, wave, narrow, s)) {
+    cudaError_t e;
+    if constexpr (W == kLanes) e = launch_persistent<DMAX>(p, s);
+    else e = launch_narrow<DMAX, W>(p, s);
     if (e == cudaSuccess) done = true;
     else if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration)
       return e;
@@ -1080,7 +1248,7 @@ cudaError_t launch_multi(LdpcMultiParams m, cudaStream_t s) {
   if ((e = cudaStreamIsCapturing(s, &cs)) != cudaSuccess) return e;
   if (cs == cudaStreamCaptureStatusNone) {
     void* args[] = {&m};
-    return ldpc_persist_launch(s, reinterpret_cast<const void*>(h2_multi<DMAX>), unsigned(blocks), kWarps * 32, args);
+    return ldpc_persist_launch(s, reinterpret_cast<const void*>(h2_multi<DMAX>), unsigned(blocks), kWarps * 32, 0, args);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(blocks));
@@ -1181,7 +1349,8 @@ cudaError_t launch_ldpc_h2_multi(LdpcMultiParams m, int d_max, cudaStream_t s) {
 cudaError_t launch_ldpc_lanes_h2(LdpcLanesParams p, void* scratch, cudaStream_t s) {
   if (p.nframes <= 0) return cudaSuccess;
   if (p.state_in || p.algorithm != 2) return cudaErrorInvalidValue;
-  const int W = ldpc_lanes_h2_width(p.nframes);
+  int W = ldpc_lanes_h2_width(p.nframes);
+  if (W < 4 && persists_alone(p)) W = 4;
   ldpc_lanes_h2_layout(p, scratch, W);
   if (p.d_max <= 8) return run_width<8>(p, W, s);
   if (p.d_max <= 16) return run_width<16>(p, W, s);

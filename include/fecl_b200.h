@@ -317,9 +317,11 @@ int fecl_ldpc_set_wave(fecl_codec_t codec, int32_t groups);
 
 /* Lane-batched LDPC decoder: run a small batch (at most 16 frame groups, one wave)
  * as one persistent launch whose check and bit passes are separated by grid-wide
- * barriers, instead of two launches per iteration.  mode 1: wherever it applies;
- * 0 (the built-in choice) and -1: never -- the per-pass launches, which overlap their
- * launch latency through programmatic dependent launch, measured faster.  The
+ * barriers, instead of two launches per iteration.  mode 1: wherever it applies; -1:
+ * never; 0 (the built-in choice): for up to 16 frames of a code of at most 20000 bits with
+ * packed FP16 messages, decoded by a call of their own (not in a mixed batch, the server,
+ * or a stream capture), which it measured faster on; otherwise the per-pass launches,
+ * which overlap their launch latency through programmatic dependent launch.  The
  * results are those of the two-launch form bit for bit.  A barrier wait is bounded
  * (2 s); a decode whose barrier gave up reports -1 iterations for its frames.
  * Extension: no counterpart in the reference. */

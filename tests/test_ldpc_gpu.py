@@ -499,3 +499,30 @@ def test_in_place_fp32_messages_equal_the_persistent_launch(alg, n, rate, frames
     code.setPersistent(1)
     for a, b in zip(mine, everything()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,rate", [(16200, (1, 2)), (16200, (8, 9)), ("gallager", None)])
+def test_small_batches_in_one_launch_equal_a_launch_per_pass(n, rate):
+    """1 to 16 FP16 frames, which take the persistent launch by themselves, against a launch
+    per pass (mode -1): bits, iteration counts and soft outputs equal, for frames that
+    retire apart or never."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    H = F.Ldpc.Gallager.matrix(2048, 3, 5, 0) if n == "gallager" else F.Ldpc.DvbS2.matrix(n, Fraction(*rate))
+    opts = F.Ldpc.DecoderOptions().algorithm(F.Approximate).iterations(20).scalingFactor(0.75).precision(1)
+    for fixed in (False, True):
+        code = F.Ldpc(F.Ldpc.EncoderOptions(H), opts.fixedIterations(fixed))
+        K, N = code.msgSize(), code.paritySize()
+        for frames in (1, 3, 5, 8, 9, 16, 17):
+            msg = ch.random_bits(frames * K, 92)
+            llr = torch.from_numpy(ch.awgn_llr_per_frame(code.encode(msg), N, np.linspace(7.0, 0.5, frames), K / N, 92,
+                                                         np.float32)).cuda()
+            got = []
+            for mode in (0, -1):
+                code.setPersistent(mode)
+                bits, its = code.decode(llr, iterations=True)
+                out = code.soDecode(F.Codec.Input().parity(llr), F.Codec.Output(np.float32).msg().parity().state())
+                got.append((bits, its, out.msg(), out.parity(), out.state()))
+            assert all(torch.equal(a, b) for a, b in zip(*got)), (frames, fixed)
+            assert int(got[0][1].min()) > 0
