@@ -256,8 +256,21 @@ __device__ __forceinline__ uint32_t* signs_of(const LdpcLanesParams& p, int g) {
 template <int ALG, int DMAX>
 constexpr int flow_rows() { return DMAX <= 8 && ALG == kApproximate ? 2 : 1; }
 
+// Blocks per SM that the registers have to leave room for: the pass waits for L2 and for the
+// transforms' chains.  Without these bounds (136 registers for a Linear row of up to 16, one
+// block per SM) and with them, 64 frames: Linear short r=3/5 2977 and 1568 us, r=8/9 1335 and
+// 886, normal r=9/10 3826 and 2079; Exact short r=3/5 2088 and 1425; min-sum short r=1/2 735 and
+// 691 (482 and 420 for 5 frames, whose blocks now fit one wave), r=3/5 745 and 725.  A block
+// more or less in each class was slower, in Exact by the spills.
 template <int ALG, int DMAX>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, ALG == kApproximate ? (DMAX > 16 ? 3 : 1) : (DMAX <= 8 ? 4 : 1)) flow_check(LdpcLanesParams p, int it, int g0) {
+constexpr int flow_blocks() {
+  if (ALG == kApproximate) return DMAX <= 8 ? 4 : DMAX <= 16 ? 4 : 3;
+  if (ALG == kExact) return DMAX <= 8 ? 4 : DMAX <= 16 ? 2 : 1;
+  return DMAX <= 8 ? 4 : DMAX <= 16 ? 4 : 3;
+}
+
+template <int ALG, int DMAX>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, flow_blocks<ALG, DMAX>()) flow_check(LdpcLanesParams p, int it, int g0) {
   pdl_enter();
   constexpr int kRows = flow_rows<ALG, DMAX>();
   const int lane = lane_id();
@@ -748,11 +761,20 @@ cudaError_t run_flow(const LdpcLanesParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// One group of short frames with Linear rows of 9 to 16 edges keeps the a-posteriori values: the
+// table's chains bound its check pass, so the in-place bit pass's stores are not won back (32
+// DVB-S2 short frames, a-posteriori values and in place: r=3/5 715 and 777 us, r=2/3 622 and 666;
+// more groups or 64800 bits are up to 15 % faster in place, r=3/5 with 64 frames 3 % slower).
+template <int ALG, int DMAX>
+bool keeps_app(const LdpcLanesParams& p) {
+  return ALG == kLinear && DMAX == 16 && p.groups == 1 && p.N <= 20000;
+}
+
 template <int ALG, int MSG, int DMAX>
 cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   if (p.groups > 65535) return cudaErrorInvalidValue;
   if constexpr (MSG == 0)
-    if (p.persist <= 0) return run_flow<ALG, DMAX>(p, s);
+    if (p.persist <= 0 && !keeps_app<ALG, DMAX>(p)) return run_flow<ALG, DMAX>(p, s);
   const int wave = wave_for(p, group_bytes(p));
   const dim3 gs((148 * 8 + p.groups - 1) / p.groups, p.groups);
   lanes_stage<MSG><<<gs, 256, 0, s>>>(p);

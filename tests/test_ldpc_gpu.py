@@ -467,7 +467,8 @@ def test_in_place_messages_equal_the_soft_path(n, rate, frames):
 
 
 @pytest.mark.parametrize("alg,n,rate,frames", [(0, 16200, (1, 2), 33), (1, 16200, (4, 5), 31), (2, 16200, (8, 9), 65),
-                                               (2, 64800, (3, 5), 40), (2, "gallager", None, 70)])
+                                               (2, 64800, (3, 5), 40), (2, "gallager", None, 70),
+                                               (1, 16200, (2, 3), 32), (1, 16200, (2, 3), 33)])
 def test_in_place_fp32_messages_equal_the_persistent_launch(alg, n, rate, frames):
     """FP32 messages turned around in place against the persistent launch, which keeps the
     a-posteriori values: bits, iteration counts and every soft output equal, with frames
