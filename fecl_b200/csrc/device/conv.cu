@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(kEncodeThreads) conv_encode_cta(const __grid_c
   encode_constituent(c, msg + f * c.msg_size, nullptr, parity + f * c.parity_size, nullptr, sh, s);
 }
 
-// A thread per frame, for trellises and lengths beyond conv_encode_cta's.
+// A thread per frame, for trellises and lengths beyond conv_encode_cta's and for many short messages
+// (encode_cta_us).
 __global__ void conv_encode_kernel(TurboDeviceConstituent c, const uint8_t* msg, uint8_t* parity, int64_t nframes) {
   const int64_t f = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (f >= nframes) return;
@@ -387,7 +388,7 @@ cudaError_t launch_viterbi(const TurboDeviceConstituent& k, const ViterbiRun& r,
 cudaError_t launch_conv_encode(const TurboDeviceConstituent& c, const uint8_t* msg, uint8_t* parity, int64_t nframes,
                                cudaStream_t s) {
   if (nframes <= 0) return cudaSuccess;
-  if (encode_by_cta(c) && nframes <= 0x7fffffff) {
+  if (encode_by_cta(c) && nframes <= 0x7fffffff && encode_cta_us(c, nframes) <= encode_thread_us(c, nframes, 200.0)) {
     const cudaError_t e = cudaFuncSetAttribute(conv_encode_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, c.length);
     if (e != cudaSuccess) return e;
     conv_encode_cta<<<unsigned(nframes), kEncodeThreads, size_t(c.length), s>>>(c, msg, parity);

@@ -21,6 +21,8 @@
 #include "kernels.hpp"
 #include "trellis_encode.cuh"
 
+#include <algorithm>
+
 namespace fecl {
 namespace {
 
@@ -273,7 +275,8 @@ __global__ void __launch_bounds__(kEncodeThreads) turbo_encode_cta(const __grid_
   encode_constituent(code.c[j], m, code.c[j].perm, out + par, out + tail, sh, s);
 }
 
-// Thread (frame, constituent j), for trellises and lengths beyond turbo_encode_cta's;
+// Thread (frame, constituent j), for trellises and lengths beyond turbo_encode_cta's and for many
+// short messages (encode_cta_us);
 // constituent 0's thread also copies the message.
 __global__ void turbo_encode_kernel(TurboDeviceCode code, const uint8_t* msg, uint8_t* parity, int64_t nframes) {
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -418,11 +421,14 @@ cudaError_t launch_turbo_encode(const TurboDeviceCode& code, const uint8_t* msg,
   if (nframes <= 0) return cudaSuccess;
   bool by_cta = nframes * code.n <= 0x7fffffff;
   int longest = 0;
+  double cta = 0.0, thread = 0.0;
   for (int j = 0; j < code.n; ++j) {
     by_cta = by_cta && encode_by_cta(code.c[j]);
+    cta += encode_cta_us(code.c[j], nframes);
+    thread = std::max(thread, encode_thread_us(code.c[j], nframes * code.n, 400.0));
     longest = code.c[j].length > longest ? code.c[j].length : longest;
   }
-  if (by_cta) {
+  if (by_cta && cta <= thread) {
     const cudaError_t e = cudaFuncSetAttribute(turbo_encode_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, longest);
     if (e != cudaSuccess) return e;
     turbo_encode_cta<<<unsigned(nframes * code.n), kEncodeThreads, size_t(longest), s>>>(code, msg, parity);

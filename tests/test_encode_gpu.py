@@ -113,10 +113,11 @@ def test_ldpc_encoder_frames_per_cta_and_alignment(code, frames):
         assert torch.equal(c.encode(buf[offset:]), want), offset
 
 
-@pytest.mark.parametrize("K,frames", [(1, 2), (40, 300), (127, 3), (128, 2), (129, 2), (6144, 5)])
+@pytest.mark.parametrize("K,frames", [(1, 2), (40, 300), (127, 3), (128, 2), (129, 2), (6144, 5),
+                                      (40, 4000), (129, 1500)])
 def test_trellis_encoders_by_chunks(K, frames):
-    """One step, chunks of one step (threads without any), a chunk more than the threads;
-    4 to 64 states, one and two inputs, one to three outputs.  Bits: equal to the host's."""
+    """One step, chunks of one step (threads without any), a chunk more than the threads,
+    many short messages (a thread each); 4 to 64 states, one and two inputs, one to three outputs.  Bits: equal to the host's."""
     import torch
     import fecl_b200 as F
     from fecl_b200 import channel as ch
