@@ -214,8 +214,8 @@ int fecl_conv_puncturing(fecl_codec_t codec, const uint8_t* mask, uint32_t mask_
 int fecl_codec_sizes(fecl_codec_t codec, fecl_sizes* sizes);
 
 /* Codec::encode -- src/Codec.h:171-198.  Bits are one byte each (0/1).  With
- * FECL_DEVICE_MEMORY the frames are encoded on the GPU (one thread per frame, the
- * reference's encoding steps, bit-exact), asynchronously on `stream`. */
+ * FECL_DEVICE_MEMORY the frames are encoded on the GPU (the reference's
+ * encoding steps, bit-exact), asynchronously on `stream`. */
 int fecl_encode(fecl_codec_t codec, const uint8_t* msg, uint64_t nframes, uint8_t* parity, int32_t flags,
                 void* stream);
 
@@ -293,8 +293,7 @@ void fecl_permutation_destroy(fecl_permutation_t perm);
 
 /* Kernel selection: FECL_KERNEL_AUTO picks the fastest kernel that supports the
  * code and options; FECL_KERNEL_GENERIC forces the generic kernels, which walk the
- * reference's operation order in FP32 (one thread per turbo frame, one CTA per
- * LDPC frame). */
+ * reference's operation order in FP32 (a CTA per frame). */
 #define FECL_KERNEL_AUTO 0
 #define FECL_KERNEL_GENERIC 1
 /* LDPC only: the lane-batched decoder (32 frames per warp, messages in device
