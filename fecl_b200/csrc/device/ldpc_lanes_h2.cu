@@ -455,8 +455,11 @@ constexpr int kFlowBits = 2;
 
 // Bit pass after the check pass of iteration `it`, or with it < 0 the first one.  Block (0, y)
 // retires frames, as in h2_bit; a group none of whose frames goes on keeps its messages.
+// Four blocks per SM: the compiler alone took 66 registers with whole warps per bit, three
+// blocks (64 DVB-S2 normal r=1/2 frames 1318 and 1204 us, 512 of r=3/4 5.73 and 5.34 ms; five
+// blocks cost r=9/10 5 %).  Narrower groups need 40.
 template <int W>
-__global__ void __launch_bounds__(kWarps * 32) flow_bit(LdpcLanesParams p, int it, int g0) {
+__global__ void __launch_bounds__(kWarps * 32, W == 32 ? 4 : 0) flow_bit(LdpcLanesParams p, int it, int g0) {
   pdl_enter();
   constexpr int kSlots = 32 / W;
   constexpr uint32_t kAll = W == 32 ? 0xffffffffu : (1u << W) - 1u;
