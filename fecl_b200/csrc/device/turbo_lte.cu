@@ -1263,9 +1263,15 @@ size_t turbo_lte_scratch_bytes(int K, int64_t nframes, bool extra) {
     positions = std::max(positions, g.perm_floats());
   }
   const int Tp = LteGeometry(K, kDefaultSegs).Tp;
-  return (size_t(nframes) * (size_t(frame) + (extra ? size_t(3 * Tp) : 0)) +
-          size_t(nframes <= kStageHere ? nframes + 1 : 2) * size_t(positions)) *
-         sizeof(float);
+  auto need = [&](int64_t n) {
+    return (size_t(n) * (size_t(frame) + (extra ? size_t(3 * Tp) : 0)) +
+            size_t(n <= kStageHere ? n + 1 : 2) * size_t(positions)) *
+           sizeof(float);
+  };
+  // never less than a smaller batch takes: a host call's chunks share the plan of the longest, and
+  // a last one of at most kStageHere frames holds positions for each (148 frames of K = 6144
+  // take more than 149)
+  return std::max(need(nframes), need(std::min(nframes, kStageHere)));
 }
 
 cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
