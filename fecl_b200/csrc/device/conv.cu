@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(32) viterbi_warp(TurboDeviceConstituent k, Vit
       odd = odd || !isfinite(x);
     }
     infinite = __any_sync(0xffffffffu, odd) || infinite;
+    __syncwarp();  // the block's L-values, other lanes' among them (a vote does not order memory)
     for (int e = sub; e < kStep * O; e += G) {
       const int t = e >> os, o = e & (O - 1);
       double x = 0.0;

@@ -74,3 +74,21 @@ def test_viterbi_lanes_match_the_reference_loops(code, length, frames):
         want = viterbi(tr, c.msgSize() // int(np.log2(tr.inputCount())), T - c.msgSize() // int(np.log2(tr.inputCount())),
                        term, finite.astype(np.float64))
         assert np.array_equal(c.decode(finite), want), (code, term, "f16")
+
+
+# three and more outputs per step: a lane loads more of a block's L-values than it keeps ahead, and
+# every branch metric adds values that other lanes stored
+@pytest.mark.parametrize("spec,length,frames", [
+    (([3], [[0o7, 0o5, 0o6]], None), 100, 17), (([4], [[0o15, 0o17, 0o13, 0o11]], None), 97, 9),
+    (([6], [[0o53, 0o75, 0o61]], None), 131, 3), (([7], [[0o171, 0o133, 0o165]], None), 200, 5),
+    (([7], [[0o171, 0o133, 0o165, 0o117, 0o155, 0o127]], [0o147]), 65, 3)])
+def test_viterbi_lanes_share_a_block_of_many_outputs(spec, length, frames):
+    import fecl_b200 as F
+    tr = F.Trellis(*spec)
+    for term in (0, 1):
+        c = F.Convolutional(F.Convolutional.EncoderOptions(tr, length).termination(term))
+        tail = c.paritySize() // tr.outputSize() - length
+        rng = np.random.default_rng([length, frames, term, 7])
+        word = c.encode(rng.integers(0, 2, frames * length).astype(np.uint8))
+        llr = (2.0 * (2.0 * word - 1.0) + 2.5 * rng.normal(size=word.size)).astype(np.float32)
+        assert np.array_equal(c.decode(llr), viterbi(tr, length, tail, term, llr.astype(np.float64))), term
