@@ -92,6 +92,19 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, F&& up
   return e;
 }
 
+// Lets `kern` be launched with all the dynamic shared memory that a block of this device can have
+// beside `fixed` bytes of the kernel's own.  The limit is the kernel's, not the launch's: set to what
+// one launch takes, it would refuse the larger launch that another thread makes next.  So every
+// caller of a kernel sets the same value, and none lowers it.
+template <typename... KArgs>
+inline cudaError_t allow_shared_memory(void (*kern)(KArgs...), size_t fixed = 1024) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(fixed));
+}
+
 // Programmatic dependent launch.  A kernel launched with launch_pdl may be scheduled
 // while the previous kernel of its stream is still running; pdl_enter, its first
 // statement, waits until that kernel has completed and its writes are visible (a

@@ -390,7 +390,7 @@ cudaError_t launch_conv_encode(const TurboDeviceConstituent& c, const uint8_t* m
                                cudaStream_t s) {
   if (nframes <= 0) return cudaSuccess;
   if (encode_by_cta(c) && nframes <= 0x7fffffff && encode_cta_us(c, nframes) <= encode_thread_us(c, nframes, 200.0)) {
-    const cudaError_t e = cudaFuncSetAttribute(conv_encode_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, c.length);
+    const cudaError_t e = allow_shared_memory(conv_encode_cta, kEncodeFixed);
     if (e != cudaSuccess) return e;
     conv_encode_cta<<<unsigned(nframes), kEncodeThreads, size_t(c.length), s>>>(c, msg, parity);
     return cudaGetLastError();

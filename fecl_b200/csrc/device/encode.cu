@@ -405,7 +405,7 @@ cudaError_t launch_ldpc_encode(const LdpcEncodeTables& t, const uint8_t* msg, ui
   const uintptr_t parts = uintptr_t(t.K) | uintptr_t(t.N) | uintptr_t(t.gap) | reinterpret_cast<uintptr_t>(msg) |
                           reinterpret_cast<uintptr_t>(parity);
   auto run = [&](auto kern) -> cudaError_t {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(t.bytes));
+    cudaError_t err = allow_shared_memory(kern);
     if (err != cudaSuccess) return err;
     kern<<<unsigned(blocks), threads, t.bytes, s>>>(t, msg, parity, nframes, int(per));
     return cudaGetLastError();
@@ -429,7 +429,7 @@ cudaError_t launch_turbo_encode(const TurboDeviceCode& code, const uint8_t* msg,
     longest = code.c[j].length > longest ? code.c[j].length : longest;
   }
   if (by_cta && cta <= thread) {
-    const cudaError_t e = cudaFuncSetAttribute(turbo_encode_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, longest);
+    const cudaError_t e = allow_shared_memory(turbo_encode_cta, kEncodeFixed);
     if (e != cudaSuccess) return e;
     turbo_encode_cta<<<unsigned(nframes * code.n), kEncodeThreads, size_t(longest), s>>>(code, msg, parity);
     return cudaGetLastError();

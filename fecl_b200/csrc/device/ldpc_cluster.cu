@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(THREADS, 1) ldpc_cluster_kernel(LdpcClusterPar
 template <int ALG, int MSG, int DMAX, int THREADS, bool CL>
 cudaError_t launch_one(const LdpcClusterParams& p, int clusters, size_t smem, cudaStream_t s) {
   auto kern = ldpc_cluster_kernel<ALG, MSG, DMAX, THREADS, CL>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_shared_memory(kern);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -386,7 +386,7 @@ int ldpc_cluster_max_active(const LdpcClusterParams& p) {
   const size_t smem = ldpc_cluster_smem_bytes(p.max_edges, p.max_bits, p.msg_type);
   int result = 0;
   auto query = [&](auto kern) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
+    if (allow_shared_memory(kern) != cudaSuccess) {
       cudaGetLastError();
       return;
     }

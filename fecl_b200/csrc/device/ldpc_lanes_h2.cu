@@ -1125,7 +1125,7 @@ cudaError_t launch_narrow(LdpcLanesParams p, cudaStream_t s) {
   const size_t smem = kBlockWarps * narrow_words_per_warp(p.d_max, p.c_max, W, rows, bits) * 4;
   if (blocks < 1 || smem + 1024 > size_t(limit)) return cudaErrorInvalidConfiguration;
   auto kern = h2_persist_narrow<DMAX, W>;
-  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess) return e;
+  if ((e = allow_shared_memory(kern)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
   void* args[] = {&p, &rows, &bits};
   return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kNarrowThreads, smem, args);

@@ -41,6 +41,8 @@ struct EncodeShared {
   uint8_t map[kEncodeThreads][kEncodeStates];
   uint8_t start[kEncodeThreads + 1];
 };
+constexpr size_t kEncodeFixed = sizeof(EncodeShared) + 1024;
+static_assert(kEncodeFixed + kEncodeSteps <= 227 << 10);
 
 // Message m (through the interleaver where perm is given) into the parity bits at par and,
 // where tail_out is given, the termination's input bits there.  steps: c.length bytes of shared memory.

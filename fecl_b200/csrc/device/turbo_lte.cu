@@ -1326,7 +1326,7 @@ cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
       case kF16: turbo_lte_stage<__half><<<blocks, 256, 0, s>>>(q); break;
       default: turbo_lte_stage<float><<<blocks, 256, 0, s>>>(q); break;
     }
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t err = allow_shared_memory(kern);
     if (err != cudaSuccess) return err;
     kern<<<unsigned(n), 2 * segs, smem, s>>>(q);
     return cudaGetLastError();
@@ -1372,7 +1372,7 @@ int turbo_lte_batch_max_ctas(int max_K, int algorithm, bool whole) {
   const size_t smem = lte_smem_bytes<kDefaultSegs>(max_K);
   int per_sm = 0, sms = 0, dev = 0;
   auto kern = batch_kernel(algorithm, whole);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
+  if (allow_shared_memory(kern) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 2 * kDefaultSegs, smem) != cudaSuccess) {
     cudaGetLastError();
     per_sm = 0;
@@ -1400,7 +1400,7 @@ cudaError_t launch_turbo_lte_batch(const TurboLteBatchParams& p, cudaStream_t s)
   if (ctas <= 0) return cudaErrorInvalidConfiguration;
   if (int64_t(ctas) > q.nframes) ctas = int(q.nframes);
   auto kern = batch_kernel(q.algorithm, q.whole != 0);
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  e = allow_shared_memory(kern);
   if (e != cudaSuccess) return e;
   kern<<<unsigned(ctas), 2 * kDefaultSegs, smem, s>>>(q);
   return cudaGetLastError();
