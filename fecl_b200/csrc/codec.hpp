@@ -407,7 +407,7 @@ struct fecl_codec_s {
   std::map<uint32_t, std::unique_ptr<ClusterDev>> cplans;
   int cluster_size_sel = 0, cluster_threads_sel = 0;  // 0: chosen by the heuristic
   int lanes_wave = 0;                                 // 0: chosen by the launcher
-  int lanes_persist = 0;                              // persistent launch: 1 where it applies, 0 / -1 never
+  int lanes_persist = 0;                              // persistent launch: 1 where it applies, 0 where it is the faster, -1 never
   int smem_optin = 0, sm_count = 0;
 
   ClusterDev& cluster_plan(uint32_t C) {
@@ -533,7 +533,7 @@ struct Launch {
   int32_t* iters = nullptr;
   void *msg = nullptr, *syst_out = nullptr, *parity_out = nullptr, *state_out = nullptr;
   char* scratch = nullptr;
-  bool alone = false;  // the call's only decode on the device
+  bool alone = false;  // the call's only decode (not: the only one on the device)
 };
 
 // Scratch of the decoder kernels for n frames, with the offsets of its parts.

@@ -61,7 +61,8 @@ struct LdpcLanesParams {
   int32_t msg_type = 0;  // 0 FP32, 1 FP16, 2 saturated int8 (Q5.2)
   int32_t wave_groups = 0;  // groups decoded together (0: as many as fit in 64 MiB of L2)
   // one persistent launch for small batches: 1 wherever it applies, -1 never, 0 where it is the
-  // faster and the call is `alone`: not one of several decodes launched to run beside one another
+  // faster and the call is `alone`: its only decode, not a chunk of a host batch nor a job of a mixed
+  // batch or the server, which are launched to run beside one another
   int32_t persist = 0, alone = 0;
   // batch, frame-major caller buffers
   int64_t nframes = 0;
@@ -89,8 +90,11 @@ struct LdpcLanesParams {
 
 size_t ldpc_lanes_scratch_bytes(int64_t N, int64_t E, int64_t nframes, int msg_type);
 // Cooperative launch of a persistent LDPC kernel, ordered after the previous one on
-// this device (ldpc_lanes.cu).
-cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, size_t smem, void** args);
+// this device (ldpc_lanes.cu).  asked: the caller chose the persistent form.  Where this or the previous
+// one was not asked for and the previous one is under way on another stream: cudaErrorNotReady,
+// with nothing launched and nothing waited for.
+cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, size_t smem, void** args,
+                                bool asked);
 cudaError_t launch_ldpc_lanes(LdpcLanesParams p, void* scratch, cudaStream_t stream);
 
 // Normalised min-sum with FP16 messages and packed half2 check-node arithmetic, two

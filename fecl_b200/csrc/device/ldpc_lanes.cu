@@ -699,23 +699,48 @@ bool use_persistent(const LdpcLanesParams& p, int wave, cudaStream_t s) {
 
 // Persistent launches of one device run one after the other, whatever their streams,
 // so that two of them never hold parts of the GPU while each waits for the rest: every
-// such launch waits for an event the previous one recorded.
+// such launch is ordered after an event the previous one recorded.  Only launches that the
+// callers asked for wait for one another across streams.  One that is merely the built-in choice
+// is not made, nor is one made to wait for it, while the other is under way on another stream:
+// the call takes its launches per pass, and no stream waits for one it has nothing to do with.
 namespace {
+struct PersistTail {
+  cudaEvent_t done = nullptr;
+  unsigned long long stream = 0;  // cudaStreamGetId: handles are used again, ids are not
+  bool asked = false;
+};
 std::mutex g_persist_mu;
-cudaEvent_t g_persist_ev[64] = {};
+PersistTail g_persist_tail[64];
+
+// cudaEventQuery, which a capture that another thread has begun in the global mode would not survive.
+cudaError_t query_beside_captures(cudaEvent_t ev) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return e;
+  const cudaError_t state = cudaEventQuery(ev);
+  if (state == cudaErrorNotReady) cudaGetLastError();
+  e = cudaThreadExchangeStreamCaptureMode(&mode);
+  return e != cudaSuccess ? e : state;
+}
 }  // namespace
 
-cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, size_t smem, void** args) {
+cudaError_t ldpc_persist_launch(cudaStream_t s, const void* kern, unsigned blocks, unsigned threads, size_t smem, void** args,
+                                bool asked) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lk(g_persist_mu);
-  if (!g_persist_ev[dev] && (e = cudaEventCreateWithFlags(&g_persist_ev[dev], cudaEventDisableTiming)) != cudaSuccess)
-    return e;
-  if ((e = cudaStreamWaitEvent(s, g_persist_ev[dev], 0)) != cudaSuccess) return e;
+  PersistTail& tail = g_persist_tail[dev];
+  if (!tail.done && (e = cudaEventCreateWithFlags(&tail.done, cudaEventDisableTiming)) != cudaSuccess) return e;
+  unsigned long long stream = 0;
+  if ((e = cudaStreamGetId(s, &stream)) != cudaSuccess) return e;
+  if (stream != tail.stream && !(asked && tail.asked) && (e = query_beside_captures(tail.done)) != cudaSuccess) return e;
+  if ((e = cudaStreamWaitEvent(s, tail.done, 0)) != cudaSuccess) return e;
   if ((e = cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, smem, s)) != cudaSuccess) return e;
-  return cudaEventRecord(g_persist_ev[dev], s);
+  tail.stream = stream;
+  tail.asked = asked;
+  return cudaEventRecord(tail.done, s);
 }
 
 namespace {
@@ -736,7 +761,7 @@ cudaError_t launch_persistent(LdpcLanesParams p, cudaStream_t s) {
   if (blocks < 1) return cudaErrorInvalidConfiguration;
   if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
   void* args[] = {&p};
-  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarpsPerBlock * 32, 0, args);
+  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarpsPerBlock * 32, 0, args, true);
 }
 
 // A decode with FP32 messages in place; waves as below, of the smaller working set.
@@ -782,7 +807,8 @@ cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   if (use_persistent(p, wave, s)) {
     const cudaError_t e = launch_persistent<ALG, MSG, DMAX>(p, s);
     if (e == cudaSuccess) done = true;
-    else if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration)
+    else if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration &&
+             e != cudaErrorNotReady)
       return e;
     else cudaGetLastError();
   }

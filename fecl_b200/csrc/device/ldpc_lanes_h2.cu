@@ -1068,7 +1068,8 @@ __global__ void __launch_bounds__(kWarps * 32) h2_bit_many(LdpcMultiParams m, in
 // per-pass launches are the built-in choice: see ldpc_lanes.cu).
 
 // One narrow group of a code of at most kPersistBits bits takes the persistent launch by itself
-// when its call is the only decode under way: 1 to 16 DVB-S2 short frames, 50 iterations allowed,
+// where its call decodes nothing else beside it (`alone`) and no persistent launch of another stream is under
+// way (ldpc_persist_launch): 1 to 16 DVB-S2 short frames, 50 iterations allowed,
 // took 80 to 105 us against 230 a dB above the waterfall (8 iterations), 175 to 220 against
 // 250 to 305 in it (18), and as long with frames that never converge (437 to 481 against 433 to
 // 535).  Frames of 64800 bits gained as much when they converged early but ran 8 to 20 %
@@ -1106,7 +1107,7 @@ cudaError_t launch_persistent(LdpcLanesParams p, cudaStream_t s) {
   if (blocks < 1) return cudaErrorInvalidConfiguration;
   if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
   void* args[] = {&p};
-  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarps * 32, 0, args);
+  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kWarps * 32, 0, args, true);
 }
 
 // One block per SM at most; cudaErrorInvalidConfiguration where the index lists do not fit.
@@ -1128,7 +1129,7 @@ cudaError_t launch_narrow(LdpcLanesParams p, cudaStream_t s) {
   if ((e = allow_shared_memory(kern)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(p.barrier, 0, 2 * sizeof(unsigned), s)) != cudaSuccess) return e;
   void* args[] = {&p, &rows, &bits};
-  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kNarrowThreads, smem, args);
+  return ldpc_persist_launch(s, reinterpret_cast<const void*>(kern), unsigned(blocks), kNarrowThreads, smem, args, p.persist > 0);
 }
 
 // The grid of the staging and finishing kernels: 256 threads per block over the
@@ -1195,7 +1196,8 @@ cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
     if constexpr (W == kLanes) e = launch_persistent<DMAX>(p, s);
     else e = launch_narrow<DMAX, W>(p, s);
     if (e == cudaSuccess) done = true;
-    else if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration)
+    else if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration &&
+             e != cudaErrorNotReady)
       return e;
     else cudaGetLastError();
   }
@@ -1251,7 +1253,7 @@ cudaError_t launch_multi(LdpcMultiParams m, cudaStream_t s) {
   if ((e = cudaStreamIsCapturing(s, &cs)) != cudaSuccess) return e;
   if (cs == cudaStreamCaptureStatusNone) {
     void* args[] = {&m};
-    return ldpc_persist_launch(s, reinterpret_cast<const void*>(h2_multi<DMAX>), unsigned(blocks), kWarps * 32, 0, args);
+    return ldpc_persist_launch(s, reinterpret_cast<const void*>(h2_multi<DMAX>), unsigned(blocks), kWarps * 32, 0, args, true);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(blocks));

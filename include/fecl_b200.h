@@ -319,8 +319,11 @@ int fecl_ldpc_set_wave(fecl_codec_t codec, int32_t groups);
  * barriers, instead of two launches per iteration.  mode 1: wherever it applies; -1:
  * never; 0 (the built-in choice): for up to 16 frames of a code of at most 20000 bits with
  * packed FP16 messages, decoded by a call of their own (not in a mixed batch, the server,
- * or a stream capture), which it measured faster on; otherwise the per-pass launches,
- * which overlap their launch latency through programmatic dependent launch.  The
+ * or a stream capture) while no persistent launch of another stream is under way, which it
+ * measured faster on; otherwise the per-pass launches,
+ * which overlap their launch latency through programmatic dependent launch.  Persistent
+ * launches of mode 1 run one after the other, also across streams; those of mode 0 make no
+ * stream wait for another.  The
  * results are those of the two-launch form bit for bit.  A barrier wait is bounded
  * (2 s); a decode whose barrier gave up reports -1 iterations for its frames.
  * Extension: no counterpart in the reference. */

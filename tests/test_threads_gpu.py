@@ -79,3 +79,39 @@ def test_two_codes_of_different_size(kind):
         jobs = [decode_job(F.Turbo.lte(K, F.Turbo.DecoderOptions().algorithm(F.Approximate).iterations(2)), 2, K, 4.0)
                 for K in (40, 6144) * 3]
     assert in_threads(jobs, 3000) == []
+
+
+def one_frame_codec(persistent=0):
+    import fecl_b200 as F
+    code = F.Ldpc(F.Ldpc.EncoderOptions(F.Ldpc.DvbS2.matrix(16200, Fraction(2, 3))),
+                  F.Ldpc.DecoderOptions().algorithm(F.Approximate).iterations(10).precision(1).scalingFactor(0.75))
+    code.setPersistent(persistent)
+    return code
+
+
+# modes of the persistent launch: the built-in choice on both streams, and asked for on one of them
+@pytest.mark.parametrize("first,second", [(0, 0), (0, 1), (1, 0)])
+def test_one_frame_does_not_wait_for_another_stream(first, second):
+    """A decode queued behind long work of its own stream holds up no decode of another stream."""
+    import torch
+    jobs = [decode_job(one_frame_codec(m), 1, 7 + k, 3.0) for k, m in enumerate((first, second))]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for (call, want), st in zip(jobs, streams):
+        for _ in range(2):
+            with torch.cuda.stream(st):
+                got = call()
+            st.synchronize()
+            assert torch.equal(got, want)
+    for rehearsal in (True, False):  # loading a kernel, at its first launch, waits for the GPU
+        done = [torch.cuda.Event(), torch.cuda.Event()]
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(600_000_000)  # a third of a second
+            behind = jobs[0][0]()
+            done[0].record()
+        with torch.cuda.stream(streams[1]):
+            beside = jobs[1][0]()
+            done[1].record()
+        done[1].synchronize()
+        assert rehearsal or not done[0].query(), "the second stream waited for the first"
+        torch.cuda.synchronize()
+        assert torch.equal(behind, jobs[0][1]) and torch.equal(beside, jobs[1][1])
