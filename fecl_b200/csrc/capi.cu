@@ -221,6 +221,8 @@ fecl::LdpcLanesParams lanes_params(fecl_codec_s* c, const Launch& d, uint64_t n,
   r.wave_groups = c->lanes_wave;
   r.persist = c->lanes_persist;
   r.alone = d.alone;
+  r.barrier_us = c->barrier_us;
+  r.barrier_missing = c->barrier_missing;
   r.nframes = int64_t(n);
   r.llr = d.llr;
   r.llr_dtype = in_dtype;
@@ -1054,6 +1056,17 @@ int fecl_ldpc_set_persistent(fecl_codec_t codec, int32_t mode) {
     if (mode < -1 || mode > 1) fail(FECL_EINVAL, "persistent mode must be -1, 0 or 1");
     std::lock_guard<std::mutex> lk(c->mu);
     c->lanes_persist = mode;
+  });
+}
+
+// For tests, not declared in the header: the limit of a grid barrier's wait of the one-frame
+// LDPC launch, and arrivals that it waits for in vain.
+int fecl_test_ldpc_barrier(fecl_codec_t codec, uint32_t limit_us, uint32_t missing) {
+  return guarded([&] {
+    auto c = checked(codec);
+    std::lock_guard<std::mutex> lk(c->mu);
+    c->barrier_us = limit_us;
+    c->barrier_missing = missing;
   });
 }
 

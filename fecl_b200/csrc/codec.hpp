@@ -408,6 +408,7 @@ struct fecl_codec_s {
   int cluster_size_sel = 0, cluster_threads_sel = 0;  // 0: chosen by the heuristic
   int lanes_wave = 0;                                 // 0: chosen by the launcher
   int lanes_persist = 0;                              // persistent launch: 1 where it applies, 0 where it is the faster, -1 never
+  uint32_t barrier_us = 0, barrier_missing = 0;       // LdpcLanesParams'
   int smem_optin = 0, sm_count = 0;
 
   ClusterDev& cluster_plan(uint32_t C) {

@@ -2,7 +2,7 @@
 // the grid is resident).
 //
 // The arrival counter only grows: each barrier adds gridDim.x, and `epoch` is the
-// count a block waits for.  Every wait is bounded: after kBarrierNs of global time, or
+// count a block waits for.  Every wait is bounded: after limit_ns of global time, or
 // as soon as another block has given up (the shared failure flag), the block records
 // the failure and the barrier returns false, so that the kernel ends instead of
 // waiting for a block that will never arrive.
@@ -26,11 +26,13 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned* q) {
   return v;
 }
 
-// counter and error are two words in global memory, zeroed before the launch.
-__device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned* error, unsigned& epoch) {
+// counter and error are two words in global memory, zeroed before the launch.  `missing` more
+// arrivals than there are blocks make every wait run out.
+__device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned* error, unsigned& epoch,
+                                             unsigned long long limit_ns = kBarrierNs, unsigned missing = 0) {
   __shared__ int ok;
   __syncthreads();
-  epoch += gridDim.x;
+  epoch += gridDim.x + missing;
   if (threadIdx.x == 0) {
     // the block's writes, ordered before this thread by the barrier above, are released with the arrival
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
@@ -43,7 +45,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned* error,
         good = 0;
         break;
       }
-      if (global_ns() - t0 > kBarrierNs) {
+      if (global_ns() - t0 > limit_ns) {
         atomicExch(error, 1u);
         good = 0;
         break;

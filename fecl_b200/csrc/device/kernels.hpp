@@ -64,6 +64,9 @@ struct LdpcLanesParams {
   // faster and the call is `alone`: its only decode, not a chunk of a host batch nor a job of a mixed
   // batch or the server, which are launched to run beside one another
   int32_t persist = 0, alone = 0;
+  // a grid barrier's wait in the narrow persistent launch: its limit (0: the built-in one) and the
+  // arrivals that never come, by which a test makes it run out
+  uint32_t barrier_us = 0, barrier_missing = 0;
   // batch, frame-major caller buffers
   int64_t nframes = 0;
   const void* llr = nullptr;

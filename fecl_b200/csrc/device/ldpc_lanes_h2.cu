@@ -674,10 +674,12 @@ __global__ void __launch_bounds__(kNarrowThreads) h2_persist_narrow(LdpcLanesPar
     }
   };
   unsigned epoch = 0;
+  const unsigned long long limit = p.barrier_us ? 1000ull * p.barrier_us : kBarrierNs;
+  auto together = [&] { return grid_barrier(p.barrier, p.barrier + 1, epoch, limit, p.barrier_missing); };
   bit_pass(true, true);
   // every thread follows the masks: those of the next iteration come from these and the failures
   uint32_t ax = active_of(p, 0)[0], ay = active_of(p, 0)[1];
-  bool ok = grid_barrier(p.barrier, p.barrier + 1, epoch);
+  bool ok = together();
   for (int it = 0; ok && it < p.iterations; ++it) {
     const bool check_syndrome = it > 0 && !p.fixed_iterations;
     const bool mx = (ax >> sub) & 1, my = (ay >> sub) & 1;
@@ -715,7 +717,7 @@ __global__ void __launch_bounds__(kNarrowThreads) h2_persist_narrow(LdpcLanesPar
     }
     if (lane == 0 && (bx & ax)) atomicOr(fail_of(p, it), bx & ax);
     if (lane == 0 && (by & ay)) atomicOr(fail_of(p, it) + 1, by & ay);
-    if (!(ok = grid_barrier(p.barrier, p.barrier + 1, epoch))) break;
+    if (!(ok = together())) break;
     uint32_t on_x = ax, on_y = ay;
     if (it == p.iterations - 1) on_x = on_y = 0;
     else if (check_syndrome) {
@@ -727,11 +729,9 @@ __global__ void __launch_bounds__(kNarrowThreads) h2_persist_narrow(LdpcLanesPar
     ax = on_x;
     ay = on_y;
     if ((ax | ay) == 0) break;
-    if (!(ok = grid_barrier(p.barrier, p.barrier + 1, epoch))) break;
+    if (!(ok = together())) break;
   }
-  if (!ok && blockIdx.x == 0)
-    for (int i = threadIdx.x; i < 2 * W; i += blockDim.x) p.iters_ws[i] = -1;
-}
+}  // a barrier that gave up leaves p.barrier[1] set: h2_finish_narrow decodes
 
 // ---- several codes in one launch ------------------------------------------------
 
@@ -924,14 +924,14 @@ __global__ void __launch_bounds__(256) flow_finish(LdpcLanesParams p) {
   }
 }
 
+// The outputs of group g, by block `block` of `blocks`.
 template <int W>
-__global__ void h2_finish(LdpcLanesParams p) {
+__device__ __forceinline__ void finish_group(const LdpcLanesParams& p, int g, int block, int blocks) {
   const float2* chan = reinterpret_cast<const float2*>(p.chan);
   const float2* app = reinterpret_cast<const float2*>(p.app);
   const __half2* c2v = static_cast<const __half2*>(p.c2v);
-  const int g = int(blockIdx.y);
-  const int stride = int(gridDim.x) * blockDim.x;
-  const int t0 = int(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int stride = blocks * int(blockDim.x);
+  const int t0 = block * int(blockDim.x) + int(threadIdx.x);
   const bool soft = p.msg_out || p.syst_out || p.parity_out;
   const __half2* cg = c2v + int64_t(g) * p.E * W;
   for (int i = t0; i < p.N * W; i += stride) {
@@ -973,6 +973,60 @@ __global__ void h2_finish(LdpcLanesParams p) {
   if (p.iters && t0 < 2 * W) {
     const int64_t f = int64_t(g) * 2 * W + t0;
     if (f < p.nframes) p.iters[f] = p.iters_ws[f];
+  }
+}
+
+template <int W>
+__global__ void h2_finish(LdpcLanesParams p) {
+  finish_group<W>(p, int(blockIdx.y), int(blockIdx.x), int(gridDim.x));
+}
+
+// The decode of h2_persist_narrow by one block, from the staged L-values: for a launch whose
+// grid barrier gave up.  Slow (one SM), and as good as never needed.
+template <int DMAX, int W>
+__device__ __noinline__ void decode_by_block(const LdpcLanesParams& p) {
+  constexpr int kSlots = 32 / W, kRows = rows_per_lane<DMAX, W>();
+  const int lane = threadIdx.x & 31, sub = lane % W, slot = lane / W;
+  const int warp = threadIdx.x >> 5, warps = int(blockDim.x) >> 5;
+  const bool keep_all = p.msg_out || p.syst_out || p.parity_out || p.state_out;
+  __half2* c2v = static_cast<__half2*>(p.c2v);
+  for (int64_t i = threadIdx.x; i < p.E * W; i += blockDim.x) c2v[i] = __floats2half2_rn(0.0f, 0.0f);
+  if (threadIdx.x < 2) {
+    const int64_t left = p.nframes - int64_t(threadIdx.x) * W;
+    p.active[threadIdx.x] = left >= W ? (1u << W) - 1u : (left > 0 ? (1u << left) - 1u : 0u);
+    p.fail[threadIdx.x] = 0;
+    p.fail[2 + threadIdx.x] = 0;
+  }
+  auto bits = [&](bool mx, bool my) {
+    for (int b = warp * kSlots + slot; b < p.N; b += warps * kSlots) bit_one<W>(p, 0, b, sub, mx, my);
+  };
+  __syncthreads();
+  bits(true, true);
+  __syncthreads();
+  for (int it = 0; it < p.iterations; ++it) {
+    const uint32_t ax = active_of(p, it)[0], ay = active_of(p, it)[1];
+    if ((ax | ay) == 0) break;
+    const bool check_syndrome = it > 0 && !p.fixed_iterations, mx = (ax >> sub) & 1, my = (ay >> sub) & 1;
+    uint32_t bx = 0, by = 0;
+    for (int r0 = warp * kSlots * kRows; r0 < p.M; r0 += warps * kSlots * kRows)
+      check_rows<DMAX, W>(p, it, 0, r0 + slot * kRows, sub, mx, my, keep_all, check_syndrome, bx, by);
+    if (lane == 0 && (bx & ax)) atomicOr(fail_of(p, it), bx & ax);
+    if (lane == 0 && (by & ay)) atomicOr(fail_of(p, it) + 1, by & ay);
+    __syncthreads();
+    if (threadIdx.x < 2) retire_half<W>(p, it, 0, threadIdx.x);
+    bits(mx, my);
+    __syncthreads();
+  }
+}
+
+// h2_finish after h2_persist_narrow.
+template <int DMAX, int W>
+__global__ void __launch_bounds__(256) h2_finish_narrow(LdpcLanesParams p) {
+  if (p.barrier[1] == 0u) {
+    finish_group<W>(p, 0, int(blockIdx.x), int(gridDim.x));
+  } else if (blockIdx.x == 0) {
+    decode_by_block<DMAX, W>(p);
+    finish_group<W>(p, 0, 0, 1);
   }
 }
 
@@ -1212,6 +1266,14 @@ cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
       if (e == cudaSuccess) e = launch_pdl(h2_bit<W>, gbit, dim3(kWarps * 32), s, p, it, w0);
     }
     if (e != cudaSuccess) return e;
+  }
+  if constexpr (W < kLanes) {
+    if (done) {
+      // a thread per bit and lane: fewer blocks than stage_grid's, whose many rounds of a kernel with
+      // decode_by_block's registers took 4 us more (177 and 173 us a call)
+      h2_finish_narrow<DMAX, W><<<unsigned((int64_t(p.N) * W + 255) / 256), 256, 0, s>>>(p);
+      return cudaGetLastError();
+    }
   }
   h2_finish<W><<<gs, 256, 0, s>>>(p);
   return cudaGetLastError();

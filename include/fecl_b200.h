@@ -325,7 +325,8 @@ int fecl_ldpc_set_wave(fecl_codec_t codec, int32_t groups);
  * launches of mode 1 run one after the other, also across streams; those of mode 0 make no
  * stream wait for another.  The
  * results are those of the two-launch form bit for bit.  A barrier wait is bounded
- * (2 s); a decode whose barrier gave up reports -1 iterations for its frames.
+ * (2 s).  Where one gives up, a decode of up to 32 packed FP16 frames is done once more by a single
+ * block; larger ones, which take mode 1, report -1 iterations for their frames.
  * Extension: no counterpart in the reference. */
 int fecl_ldpc_set_persistent(fecl_codec_t codec, int32_t mode);
 

@@ -527,3 +527,26 @@ def test_small_batches_in_one_launch_equal_a_launch_per_pass(n, rate):
                 got.append((bits, its, out.msg(), out.parity(), out.state()))
             assert all(torch.equal(a, b) for a, b in zip(*got)), (frames, fixed)
             assert int(got[0][1].min()) > 0
+
+
+@pytest.mark.parametrize("n,rate,frames", [(16200, "1/2", 1), (16200, "2/3", 4), (16200, "8/9", 7), (16200, "3/5", 16)])
+@pytest.mark.parametrize("fixed", [False, True])
+def test_persistent_decode_whose_barrier_gives_up(n, rate, frames, fixed):
+    """The grid barriers of the one-frame launch wait for an arrival that never comes, for a
+    millisecond: bits and iteration counts are those of the launches per pass all the same."""
+    import ctypes as C
+    import fecl_b200 as F
+    import torch
+    from fecl_b200 import _lib, channel as ch
+    code = F.Ldpc(F.Ldpc.EncoderOptions(F.Ldpc.DvbS2.matrix(n, Fraction(rate))),
+                  F.Ldpc.DecoderOptions().algorithm(F.Approximate).iterations(6).precision(1).scalingFactor(0.75).fixedIterations(fixed))
+    msg = ch.random_bits(frames * code.msgSize(), 5)
+    ebn0 = np.linspace(1.0, 6.0, frames)
+    llr = torch.from_numpy(ch.awgn_llr_per_frame(code.encode(msg), n, ebn0, code.msgSize() / n, 6, np.float32)).cuda()
+    code.setPersistent(-1)
+    want, want_it = (x.clone() for x in code.decode(llr, iterations=True))
+    code.setPersistent(0)
+    for missing in (0, 1):
+        assert C.CDLL(F.lib_path).fecl_test_ldpc_barrier(code._h, 1000, missing) == 0
+        got, it = code.decode(llr, iterations=True)
+        assert torch.equal(got, want) and torch.equal(it, want_it), missing
