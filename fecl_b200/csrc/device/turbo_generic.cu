@@ -931,14 +931,25 @@ cudaError_t turbo_generic_init() {
   });
 }
 
-// Frames whose metrics a CTA-per-frame launch holds at once: its forward and backward metrics
-// are twice a frame's forward ones, so batches beyond twice this many frames take less scratch
-// than all their forward metrics.
-static constexpr int64_t kSlice = 4096;
+// Frames that a CTA-per-frame launch of `nframes` holds the metrics of at once, `steps` bytes forward
+// and as many backward each: all of them up to 4096, but half the batch where they take more
+// than 4 GiB, so that a batch of long frames that fits with its forward metrics alone, as a
+// thread per frame needs them, still fits.  4 GiB hold 167 frames of 50000 steps of 64 states: halves
+// that leave SMs idle belong to longer frames only.
+static int64_t slice_of(size_t steps, int64_t nframes) {
+  constexpr size_t kRoom = size_t(4) << 30;
+  const int64_t fit = int64_t(kRoom / (2 * steps));
+  const int64_t half = (nframes + 1) / 2;
+  int64_t n = half > fit ? half : fit;
+  if (n > 4096) n = 4096;
+  return n < nframes ? n : nframes;
+}
+
+static size_t steps_bytes(int64_t steps, int64_t states) { return size_t(steps) * size_t(states) * sizeof(float); }
 
 size_t turbo_generic_metrics_bytes(const TurboDeviceCode& c, int64_t nframes) {
-  const size_t steps = size_t(c.max_steps) * size_t(c.max_states) * sizeof(float);
-  return c.cta_ok ? size_t(nframes < kSlice ? nframes : kSlice) * 2 * steps : size_t(nframes) * steps;
+  const size_t steps = steps_bytes(c.max_steps, c.max_states);
+  return c.cta_ok ? size_t(slice_of(steps, nframes)) * 2 * steps : size_t(nframes) * steps;
 }
 
 cudaError_t launch_turbo_generic(const TurboDeviceCode& c, const TurboRun& p, cudaStream_t s) {
@@ -956,8 +967,9 @@ cudaError_t launch_turbo_generic(const TurboDeviceCode& c, const TurboRun& p, cu
       return turbo_generic_cta<kApproximate, kSpl>;
     };
     auto kern = c.max_states > 32 ? pick(std::integral_constant<int, 2>{}) : pick(std::integral_constant<int, 1>{});
-    for (int64_t f0 = 0; f0 < p.nframes; f0 += kSlice) {
-      const int64_t n = p.nframes - f0 < kSlice ? p.nframes - f0 : kSlice;
+    const int64_t slice = slice_of(steps_bytes(c.max_steps, c.max_states), p.nframes);
+    for (int64_t f0 = 0; f0 < p.nframes; f0 += slice) {
+      const int64_t n = p.nframes - f0 < slice ? p.nframes - f0 : slice;
       kern<<<unsigned(n), kMapThreads, 0, s>>>(c, p, f0);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
@@ -973,10 +985,13 @@ cudaError_t launch_turbo_generic(const TurboDeviceCode& c, const TurboRun& p, cu
   return cudaGetLastError();
 }
 
+// Whether the trellis takes conv_map_cta.
+static bool map_by_cta(const TurboDeviceConstituent& k) { return k.pred && (k.input_count == 2 || k.input_count == 4); }
+
 size_t conv_map_scratch_bytes(const TurboDeviceConstituent& k, int64_t nframes) {
-  const int64_t T = k.length + k.tail;
-  const int64_t metrics = T * k.state_count * (k.pred && (k.input_count == 2 || k.input_count == 4) ? 2 * (nframes < kSlice ? nframes : kSlice) : nframes);
-  return (size_t(nframes) * size_t(2 * k.parity_size + k.syst_size + k.msg_size) + size_t(metrics)) * sizeof(float) + 1024;
+  const size_t steps = steps_bytes(int64_t(k.length) + k.tail, k.state_count);
+  const size_t metrics = map_by_cta(k) ? size_t(slice_of(steps, nframes)) * 2 * steps : size_t(nframes) * steps;
+  return size_t(nframes) * size_t(2 * k.parity_size + k.syst_size + k.msg_size) * sizeof(float) + metrics + 1024;
 }
 
 cudaError_t launch_conv_map(const TurboDeviceConstituent& k, ConvMapRun r, void* scratch, cudaStream_t s) {
@@ -994,7 +1009,7 @@ cudaError_t launch_conv_map(const TurboDeviceConstituent& k, ConvMapRun r, void*
   r.app = q;
   q += r.nframes * k.msg_size;
   r.alpha = q;
-  if (k.pred && (k.input_count == 2 || k.input_count == 4)) {
+  if (map_by_cta(k)) {
     auto pick = [&](auto spl) -> void (*)(TurboDeviceConstituent, ConvMapRun, int64_t) {
       constexpr int kSpl = decltype(spl)::value;
       if (r.algorithm == kExact) return conv_map_cta<kExact, kSpl>;
@@ -1002,8 +1017,9 @@ cudaError_t launch_conv_map(const TurboDeviceConstituent& k, ConvMapRun r, void*
       return conv_map_cta<kApproximate, kSpl>;
     };
     auto kern = k.state_count > 32 ? pick(std::integral_constant<int, 2>{}) : pick(std::integral_constant<int, 1>{});
-    for (int64_t f0 = 0; f0 < r.nframes; f0 += kSlice) {
-      const int64_t n = r.nframes - f0 < kSlice ? r.nframes - f0 : kSlice;
+    const int64_t slice = slice_of(steps_bytes(int64_t(k.length) + k.tail, k.state_count), r.nframes);
+    for (int64_t f0 = 0; f0 < r.nframes; f0 += slice) {
+      const int64_t n = r.nframes - f0 < slice ? r.nframes - f0 : slice;
       kern<<<unsigned(n), kMapThreads, 0, s>>>(k, r, f0);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
