@@ -16,7 +16,8 @@
 // and within an output the sums run in the reference's order -- they are not associative
 // under the Linear and Exact algorithms -- so the values are those of one thread walking the
 // reference's loops, as turbo_generic_f32 does for the codes that keep it (states with unequal
-// numbers of predecessors, interleavers with repeated indices).  Bound by the latency of the
+// numbers of predecessors, interleavers with repeated indices) and for thousands of short
+// frames (map_cta_us).  Bound by the latency of the
 // recursions' steps (shuffle, add, table sum, warp maximum; about 85 ns in Linear with the
 // step's outputs): 128 frames of a K = 1024 two-constituent code, 6 iterations, take 1.22 ms
 // against 263 ms with a thread per frame, and 3.45 ms before the number of branches was a
@@ -945,11 +946,33 @@ static int64_t slice_of(size_t steps, int64_t nframes) {
   return n < nframes ? n : nframes;
 }
 
+// Microseconds of one MAP pass over `nframes` frames of k with a CTA and with a thread per frame, to
+// within a quarter from 4 to 64 states, 3 to 130 steps and 1 to 50000 frames.  A CTA's warps
+// share a frame's steps but pay for its start; threads all run at once, each through a chain of
+// dependent steps.  So thousands of short frames go a thread each, in Linear (CTA and thread): 4 states, 3
+// steps x 50000 frames 375 and 52 us, x 5000 59 and 46, x 1000 30 and 45; 8 states, 11 steps x
+// 50000 461 and 345, x 20000 200 and 246; all trellises of more than 32 states a CTA (7 steps of 64 states x 50000
+// 988 and 2262).
+static double map_cta_us(const TurboDeviceConstituent& k, int algorithm, int64_t nframes) {
+  const double T = double(k.length + k.tail), step = (k.state_count > 32 ? 1.25 : 0.27) * (algorithm == kExact ? 2.0 : 1.0);
+  return 25.0 + 1e-3 * double(nframes) * ((k.state_count > 32 ? 11.0 : 6.3) + step * T);
+}
+static double map_thread_us(const TurboDeviceConstituent& k, int algorithm, int64_t nframes) {
+  const double work = double(k.length + k.tail) * k.state_count;
+  return 10.0 + work * (2.2 * (algorithm == kExact ? 1.25 : algorithm == kLinear ? 1.0 : 0.85) + 4e-5 * double(nframes));
+}
+
 static size_t steps_bytes(int64_t steps, int64_t states) { return size_t(steps) * size_t(states) * sizeof(float); }
+
+// Room for either form, so that a batch never takes more than a larger one, whichever they run.
+static size_t metrics_bytes(bool cta_ok, size_t steps, int64_t nframes) {
+  const size_t thread = size_t(nframes) * steps, cta = size_t(slice_of(steps, nframes)) * 2 * steps;
+  return cta_ok && cta > thread ? cta : thread;
+}
 
 size_t turbo_generic_metrics_bytes(const TurboDeviceCode& c, int64_t nframes) {
   const size_t steps = steps_bytes(c.max_steps, c.max_states);
-  return c.cta_ok ? size_t(slice_of(steps, nframes)) * 2 * steps : size_t(nframes) * steps;
+  return metrics_bytes(c.cta_ok != 0, steps, nframes);
 }
 
 cudaError_t launch_turbo_generic(const TurboDeviceCode& c, const TurboRun& p, cudaStream_t s) {
@@ -959,7 +982,12 @@ cudaError_t launch_turbo_generic(const TurboDeviceCode& c, const TurboRun& p, cu
   if (c.max_states > kMaxS) return cudaErrorInvalidValue;
   for (int j = 0; j < c.n; ++j)
     if (c.c[j].input_count > kMaxU || c.c[j].input_size > 4) return cudaErrorInvalidValue;
-  if (c.cta_ok) {  // 2 or 4 inputs
+  double cta = 0.0, thread = 0.0;
+  for (int j = 0; j < c.n; ++j) {
+    cta += map_cta_us(c.c[j], c.algorithm, p.nframes);
+    thread += map_thread_us(c.c[j], c.algorithm, p.nframes);
+  }
+  if (c.cta_ok && cta <= thread) {  // 2 or 4 inputs
     auto pick = [&](auto spl) -> void (*)(TurboDeviceCode, TurboRun, int64_t) {
       constexpr int kSpl = decltype(spl)::value;
       if (c.algorithm == kExact) return turbo_generic_cta<kExact, kSpl>;
@@ -985,13 +1013,13 @@ cudaError_t launch_turbo_generic(const TurboDeviceCode& c, const TurboRun& p, cu
   return cudaGetLastError();
 }
 
-// Whether the trellis takes conv_map_cta.
+// Whether conv_map_cta takes the trellis.
 static bool map_by_cta(const TurboDeviceConstituent& k) { return k.pred && (k.input_count == 2 || k.input_count == 4); }
 
 size_t conv_map_scratch_bytes(const TurboDeviceConstituent& k, int64_t nframes) {
   const size_t steps = steps_bytes(int64_t(k.length) + k.tail, k.state_count);
-  const size_t metrics = map_by_cta(k) ? size_t(slice_of(steps, nframes)) * 2 * steps : size_t(nframes) * steps;
-  return size_t(nframes) * size_t(2 * k.parity_size + k.syst_size + k.msg_size) * sizeof(float) + metrics + 1024;
+  return size_t(nframes) * size_t(2 * k.parity_size + k.syst_size + k.msg_size) * sizeof(float) +
+         metrics_bytes(map_by_cta(k), steps, nframes) + 1024;
 }
 
 cudaError_t launch_conv_map(const TurboDeviceConstituent& k, ConvMapRun r, void* scratch, cudaStream_t s) {
@@ -1009,7 +1037,7 @@ cudaError_t launch_conv_map(const TurboDeviceConstituent& k, ConvMapRun r, void*
   r.app = q;
   q += r.nframes * k.msg_size;
   r.alpha = q;
-  if (map_by_cta(k)) {
+  if (map_by_cta(k) && map_cta_us(k, r.algorithm, r.nframes) <= map_thread_us(k, r.algorithm, r.nframes)) {
     auto pick = [&](auto spl) -> void (*)(TurboDeviceConstituent, ConvMapRun, int64_t) {
       constexpr int kSpl = decltype(spl)::value;
       if (r.algorithm == kExact) return conv_map_cta<kExact, kSpl>;

@@ -38,3 +38,29 @@ def test_cta_per_frame_matches_the_restatement(trellis, K, frames, alg):
                                 ("parity", out.parity(), code.paritySize()), ("state", out.state(), code.stateSize())):
             assert_soft_parity(got, want[name], ok, size, what=name, exact=alg == F.Exact,
                                linear=alg == F.Linear)
+
+
+# either side of the line between a CTA and a thread per frame, and a batch that is a few frames
+@pytest.mark.parametrize("alg", [0, 1, 2])
+@pytest.mark.parametrize("frames,length", [(20000, 1), (3000, 1), (20000, 4), (30000, 13), (20000, 13)])
+def test_many_short_frames_equal_the_frames_alone(frames, length, alg):
+    import fecl_b200 as F
+    import torch
+
+    def outputs(code, x, turbo):
+        out = F.Codec.Output(np.float32).msg().syst().parity()
+        dev = torch.from_numpy(x.ravel()).cuda()
+        code.soDecode(F.Codec.Input().parity(dev), out)
+        return [np.asarray(v.cpu()).reshape(len(x), -1)
+                for v in [out.msg(), out.syst(), out.parity()] + ([code.decode(dev)] if turbo else [])]
+
+    conv = F.Convolutional(F.Convolutional.EncoderOptions(F.Trellis([3], [[0o7, 0o5]], None), length),
+                           F.Convolutional.DecoderOptions().algorithm(alg))
+    perm = np.random.default_rng(length).permutation(length).astype(np.uint32)
+    turbo = F.Turbo(F.Turbo.EncoderOptions([F.Trellis([4], [[0o17]], [0o15])], [np.arange(length, dtype=np.uint32), perm]),
+                    F.Turbo.DecoderOptions().algorithm(alg).iterations(2))
+    for code in (conv, turbo):
+        base = np.random.default_rng([length, alg]).normal(size=(7, code.paritySize())).astype(np.float32) * 2
+        which = np.arange(frames) % 7
+        for got, want in zip(outputs(code, base[which], code is turbo), outputs(code, base, code is turbo)):
+            assert np.array_equal(got, want[which])
