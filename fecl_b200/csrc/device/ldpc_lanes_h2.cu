@@ -1226,6 +1226,22 @@ cudaError_t run_flow(const LdpcLanesParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Groups of 8 lanes, a sector per access, with rows of up to 16 edges keep the a-posteriori values
+// where they fit in L2: the in-place bit pass's scattered stores then cost more than the gathers they
+// save.  20 iterations on noise, values kept and in place: DVB-S2 short r=1/2 (rows of 7) x 48 290
+// and 310 us, x 112 561 and 583, but in its waterfall 5 % the other way from there, so the line lies
+// at 20 MB; r=3/5 x 112 699 and 776; normal r=3/5 x 48 1152 and 1273, x 80 1496 and 1610, x 112, beyond
+// L2, 2168 and 2052; a single group of normal frames 0 to 13 % slower with the values kept.  Rows of
+// more than 16 edges gain in place at every size (short r=8/9 x 48 338 and 278), and so do the jobs
+// of a mixed batch, which share L2.
+template <int DMAX, int W>
+bool keeps_app(const LdpcLanesParams& p) {
+  if (W > 8 || DMAX > 16 || !p.alone) return false;
+  const int64_t bytes = int64_t(p.groups) * W * (2 * 8 * int64_t(p.N) + 4 * p.E);
+  if (DMAX <= 8) return p.groups > 1 && bytes <= 20000000;
+  return (p.groups > 1 || p.N <= kPersistBits) && bytes <= kWaveCap;
+}
+
 template <int DMAX, int W>
 cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   if (p.groups > 65535) return cudaErrorInvalidValue;
@@ -1234,7 +1250,7 @@ cudaError_t run(const LdpcLanesParams& p, cudaStream_t s) {
   // scattered stores cost more than the gathers they save (one DVB-S2 short frame: 0.33 ms
   // against 0.25).
   if constexpr (W >= 8)
-    if (!persists_alone(p) && p.hard && !p.msg_out && !p.syst_out && !p.parity_out && !p.state_out && !p.syst_in && p.persist <= 0)
+    if (!persists_alone(p) && !keeps_app<DMAX, W>(p) && p.hard && !p.msg_out && !p.syst_out && !p.parity_out && !p.state_out && !p.syst_in && p.persist <= 0)
       return run_flow<DMAX, W>(p, s);
   constexpr int kSlots = 32 / W;
   const int64_t gb = int64_t(W) * (2 * 8 * int64_t(p.N) + 4 * p.E);

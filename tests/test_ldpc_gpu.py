@@ -550,3 +550,29 @@ def test_persistent_decode_whose_barrier_gives_up(n, rate, frames, fixed):
         assert C.CDLL(F.lib_path).fecl_test_ldpc_barrier(code._h, 1000, missing) == 0
         got, it = code.decode(llr, iterations=True)
         assert torch.equal(got, want) and torch.equal(it, want_it), missing
+
+
+# sizes on either side of the lines between messages in place and a-posteriori values kept: groups
+# of 8 lanes, one to thirteen of them, rows of up to 8, 16 and 32 edges
+@pytest.mark.parametrize("n,rate,frames", [(16200, (1, 2), 33), (16200, (1, 2), 80), (16200, (1, 2), 112),
+                                           (16200, (3, 5), 48), (16200, (3, 5), 200), (16200, (8, 9), 48),
+                                           (64800, (1, 2), 33), (64800, (3, 5), 12), (64800, (3, 5), 80),
+                                           (64800, (3, 5), 112), ("gallager", None, 48)])
+def test_both_forms_of_the_passes_decide_alike(n, rate, frames):
+    """FP16 hard decisions of a batch against those of its frames in batches of 17, which take
+    groups of 16 lanes with messages in place."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    H = F.Ldpc.Gallager.matrix(2048, 3, 5, 0) if n == "gallager" else F.Ldpc.DvbS2.matrix(n, Fraction(*rate))
+    code = F.Ldpc(F.Ldpc.EncoderOptions(H),
+                  F.Ldpc.DecoderOptions().algorithm(F.Approximate).iterations(9).scalingFactor(0.75).precision(1))
+    K, N = code.msgSize(), code.paritySize()
+    ebn0 = np.random.default_rng(frames).uniform(0.5, 6.0, frames)  # frames that retire apart or never
+    msg = ch.random_bits(frames * K, 93)
+    llr = torch.from_numpy(ch.awgn_llr_per_frame(code.encode(msg), N, ebn0, K / N, 93, np.float32)).cuda()
+    bits, its = code.decode(llr, iterations=True)
+    again = llr.reshape(frames, N)[torch.arange((frames + 16) // 17 * 17, device="cuda") % frames].reshape(-1, 17 * N)
+    parts = [code.decode(x.contiguous().view(-1), iterations=True) for x in again]
+    assert torch.equal(bits, torch.cat([b for b, _ in parts])[:frames * K])
+    assert torch.equal(its, torch.cat([i for _, i in parts])[:frames])
