@@ -576,3 +576,24 @@ def test_both_forms_of_the_passes_decide_alike(n, rate, frames):
     parts = [code.decode(x.contiguous().view(-1), iterations=True) for x in again]
     assert torch.equal(bits, torch.cat([b for b, _ in parts])[:frames * K])
     assert torch.equal(its, torch.cat([i for _, i in parts])[:frames])
+
+
+@pytest.mark.parametrize("n,rate,frames", [(16200, (1, 2), 5), (16200, (1, 2), 64), (16200, (1, 2), 65), (16200, (3, 5), 32),
+                                           (16200, (3, 5), 33), (64800, (1, 2), 33)])
+def test_linear_forms_decide_alike(n, rate, frames):
+    """Linear with FP32 messages on either side of the line between a-posteriori values kept and
+    messages in place, against the persistent launch, which keeps them."""
+    import torch
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    code = F.Ldpc(F.Ldpc.EncoderOptions(F.Ldpc.DvbS2.matrix(n, Fraction(*rate))),
+                  F.Ldpc.DecoderOptions().algorithm(F.Linear).iterations(9))
+    K, N = code.msgSize(), code.paritySize()
+    msg = ch.random_bits(frames * K, 94)
+    llr = torch.from_numpy(ch.awgn_llr_per_frame(code.encode(msg), N, np.linspace(0.5, 6.0, frames), K / N, 94, np.float32)).cuda()
+    got = []
+    for mode in (0, 1):
+        code.setPersistent(mode)
+        out = code.soDecode(F.Codec.Input().parity(llr), F.Codec.Output(np.float32).msg().syst().parity().state())
+        got.append([*code.decode(llr, iterations=True), out.msg(), out.syst(), out.parity(), out.state()])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
