@@ -1030,7 +1030,7 @@ __device__ __forceinline__ void stage_positions(const uint32_t* perm, uint16_t* 
 }
 
 // A CTA's own staging of its frame and of positions for it alone (launches of at most one frame
-// per SM, which this saves the staging launch).
+// per SM, which this saves the staging launch; kStageHere).
 __device__ __noinline__ void stage_here(const TurboLteParams& p, int64_t f, float* out, uint16_t* positions, LteMap m) {
   const int K = p.K;
   const int64_t in0 = f * int64_t(3 * K + 12), sys0 = f * int64_t(K + 6);
@@ -1192,8 +1192,13 @@ size_t lte_smem_bytes(int max_K) {
   return size_t(2 * LteGeometry(max_K, SEGS).Kp) * sizeof(float) + sizeof(Shared<SEGS>);
 }
 
-// Frames that CTAs may stage themselves (one per SM of a 148-SM GPU).
+// Frames that CTAs may stage themselves (one per SM of a 148-SM GPU), with at most so many elements
+// per thread: longer frames are staged by a launch of their own, which keeps more loads in flight than
+// the few threads of a decoding CTA.  Itself and by a launch, max-log: K=2112 decode (25 a thread) 125.8 and 123.7 us,
+// K=6144 (72) 174.8 and 167.4, K=1024 (12) the same either way; soDecode with its 128 threads K=1024
+// (24) 124.7 and 124.4, K=2112 (50) 165.7 and 157.7, K=6144 (144) 314.9 and 285.4.
 constexpr int64_t kStageHere = 148;
+constexpr int kStageElements = 24;
 
 int resolve_segs(int segs) { return segs == 32 || segs == 64 || segs == 128 ? segs : kDefaultSegs; }
 
@@ -1318,7 +1323,7 @@ cudaError_t launch_turbo_lte(TurboLteParams p, cudaStream_t s) {
     q.ynew = (p.parallel || p.soft) ? at : nullptr;
     if (q.ynew) at += n * int64_t(3 * g.Tp);
     q.perm_pos = reinterpret_cast<uint4*>(at);
-    q.stage_here = p.nframes <= kStageHere && p.nframes <= sms;
+    q.stage_here = p.nframes <= kStageHere && p.nframes <= sms && 3 * g.Tp <= kStageElements * 2 * segs;
     at += (q.stage_here ? n : 1) * int64_t(g.perm_floats());
     const unsigned blocks = unsigned(n < 148 * 8 ? n : 148 * 8) + 1;
     if (!q.stage_here) switch (p.llr_dtype) {

@@ -370,3 +370,28 @@ def test_windowed_staging_and_narrow_shapes(K, frames, alg):
         assert_hard_parity(other, ref, msg, K)
         if K <= 80:  # every segment is walked from the frame's ends
             assert np.array_equal(other, got), segs
+
+
+@pytest.mark.parametrize("K,alg", [(40, 2), (1008, 1), (1024, 1), (1024, 2), (2112, 2), (6144, 2)])
+def test_soft_frames_alone_equal_the_same_in_a_batch(K, alg):
+    """soDecode of a few frames, staged by their CTAs up to K = 1008 and by a launch beyond, against
+    the same frames in a batch that a launch stages, whose segments are the same: equal bits."""
+    import fecl_b200 as F
+    import torch
+    from fecl_b200 import channel as ch
+    code = F.Turbo.lte(K, F.Turbo.DecoderOptions().algorithm(alg).iterations(3))
+    N, frames = code.paritySize(), 149
+    llr = ch.awgn_llr(code.encode(ch.random_bits(frames * K, K)), 1.5, K / N, K, np.float32)
+    rng = np.random.default_rng(K)
+    syst = rng.normal(size=frames * code.systSize()).astype(np.float32) * 0.3
+    state = rng.normal(size=frames * code.stateSize()).astype(np.float32) * 0.3
+
+    def outputs(n):
+        inp = F.Codec.Input().parity(torch.from_numpy(llr[:n * N]).cuda())
+        inp.syst(torch.from_numpy(syst[:n * code.systSize()]).cuda()).state(torch.from_numpy(state[:n * code.stateSize()]).cuda())
+        out = code.soDecode(inp, F.Codec.Output(np.float32).msg().syst().parity().state())
+        return [v.reshape(n, -1) for v in (out.msg(), out.syst(), out.parity(), out.state())]
+
+    batch = outputs(frames)
+    for n in (1, 5):
+        assert all(torch.equal(a, b[:n]) for a, b in zip(outputs(n), batch))
