@@ -395,3 +395,24 @@ def test_soft_frames_alone_equal_the_same_in_a_batch(K, alg):
     batch = outputs(frames)
     for n in (1, 5):
         assert all(torch.equal(a, b[:n]) for a, b in zip(outputs(n), batch))
+
+
+@pytest.mark.parametrize("K", [8, 41, 48, 100, 1024])
+@pytest.mark.parametrize("iterations", [1, 3])
+def test_soft_max_log_equals_the_generic_kernel(K, iterations):
+    """Max-log soDecode of the LTE constituents, K a multiple of 8 (blocks without per-step tests up to
+    the last iteration) and not, against the generic kernel: 1e-4 relative, absolute below 1."""
+    import fecl_b200 as F
+    from fecl_b200 import channel as ch
+    perm = np.random.default_rng(K).permutation(K).astype(np.uint32)
+    code = F.Turbo(F.Turbo.EncoderOptions([F.Trellis([4], [[0o15]], [0o13])], [np.arange(K, dtype=np.uint32), perm]),
+                   F.Turbo.DecoderOptions().algorithm(F.Approximate).iterations(iterations))
+    frames = 5
+    llr = ch.awgn_llr(code.encode(ch.random_bits(frames * K, K)), 2.0, K / code.paritySize(), K, np.float32)
+    got = []
+    for kernel in ("auto", "generic"):
+        code.setKernel(kernel)
+        out = code.soDecode(F.Codec.Input().parity(llr), F.Codec.Output(np.float32).msg().syst().parity().state())
+        got.append([np.asarray(v) for v in (out.msg(), out.syst(), out.parity(), out.state())])
+    for a, b in zip(*got):
+        assert np.all(np.abs(a - b) <= 1e-4 * np.maximum(1.0, np.abs(b)))
