@@ -34,7 +34,8 @@
 // L2 traffic and its latency: 16 bytes per edge and lane and 8 per bit, against 20 and 16 with
 // the a-posteriori values stored, three dependent loads less per check row, and 46 MB instead of 62
 // MB per group of DVB-S2 normal frames, so that a wave holds two.  The values are the same
-// bit for bit.  DVB-S2 normal r=3/4 x 512, <= 50 iterations: 6.0 ms against 8.7.
+// bit for bit.  DVB-S2 normal r=3/4 x 512, <= 50 iterations: 5.4 ms against 8.7.  Groups of 2 or 4
+// lanes, and some batches in groups of 8 (keeps_app), keep the a-posteriori values.
 #include <cuda_fp16.h>
 #include <math.h>
 
@@ -1117,9 +1118,9 @@ __global__ void __launch_bounds__(kWarps * 32) h2_bit_many(LdpcMultiParams m, in
   for (int b = int(blockIdx.x) * kWarps + (threadIdx.x >> 5); b < p.N; b += warps) bit_one(p, g, b, lane, mx, my);
 }
 
-// One persistent launch when asked for (persist == 1) for batches of at most
-// kPersistGroups groups, all in one wave, on a stream that is not capturing (the
-// per-pass launches are the built-in choice: see ldpc_lanes.cu).
+// The persistent launches: for batches of at most kPersistGroups groups, all in one wave, on a
+// stream that is not capturing.  Where asked for (persist == 1) they take full groups of 32 lanes
+// or one narrow group; by themselves the narrow groups of persists_alone.
 
 // One narrow group of a code of at most kPersistBits bits takes the persistent launch by itself
 // where its call decodes nothing else beside it (`alone`) and no persistent launch of another stream is under

@@ -8,7 +8,7 @@
 // how it computes it is B200-shaped:
 //
 //   One CTA of 2 * SEGS threads decodes one frame for all iterations.  The frame's
-//   two exchange arrays live in shared memory in natural bit order:
+//   two exchange arrays live in shared memory by natural bit index (LteMap::pos):
 //     X[k] = Ls[k] + e0[k]          (a-priori of constituent 1 before interleaving;
 //                                    also the partial a-posteriori sum)
 //     Y[k] = e1 at natural index k  (constituent 1 writes e1(t) to Y[pi(t)])
