@@ -302,7 +302,7 @@ struct fecl_codec_s {
     tdev.parity = int32_t(turbo->parity_size());
     tdev.state = int32_t(turbo->state_size());
     tdev.tail = int32_t(turbo->syst_tail_size());
-    tdev.max_steps = 0;
+    tdev.max_steps = 1;  // at least: a truncated code of no bits has no steps, and scratch divides by their bytes
     tdev.cta_ok = 1;
     tdev.max_states = 0;
     for (size_t j = 0; j < cs.size(); ++j) {
@@ -331,7 +331,8 @@ struct fecl_codec_s {
         }
         seen[i] = true;
       }
-      if (!k.pred || c.trellis.output_size > 6 || (k.input_count != 2 && k.input_count != 4)) tdev.cta_ok = 0;
+      if (!k.pred || c.trellis.output_size > 6 || (k.input_count != 2 && k.input_count != 4) || c.length + c.tail == 0)
+        tdev.cta_ok = 0;
       tdev.max_steps = std::max(tdev.max_steps, int32_t(c.length + c.tail));
       tdev.max_states = std::max(tdev.max_states, int32_t(c.trellis.state_count));
     }

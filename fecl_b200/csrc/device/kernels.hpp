@@ -208,7 +208,7 @@ struct TurboDeviceCode {
   TurboDeviceConstituent c[kMaxConstituents];
   const float* sf = nullptr;  // [n][iterations] resolved scaling
   int32_t algorithm = 1, iterations = 6, scheduling = 0;
-  // every constituent has a predecessor table and an interleaver of distinct indices: a CTA decodes a frame
+  // every constituent has a predecessor table, an interleaver of distinct indices and a step: a CTA may decode a frame
   int32_t cta_ok = 0;
   // Custom scheduling: stage s holds activations [stage_ptr[s], stage_ptr[s+1]);
   // activation a decodes constituent act_con[a] with a-priori input from the

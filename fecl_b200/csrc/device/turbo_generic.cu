@@ -82,6 +82,7 @@ __device__ void map_pass(const TurboDeviceConstituent& k, const float* par, floa
                          float* alpha, float* app_out = nullptr) {
   const int S = k.state_count, U = k.input_count;
   const int T = k.length + k.tail;
+  if (T == 0) return;  // a truncated code of no bits: no step, no metrics
   // forward, MapDecoderImpl.cpp:117-139 (recursive) and :237-274 (LogSum)
   alpha[0] = 0.0f;
   for (int s = 1; s < S; ++s) alpha[s] = kNegInf;

@@ -64,3 +64,20 @@ def test_many_short_frames_equal_the_frames_alone(frames, length, alg):
         which = np.arange(frames) % 7
         for got, want in zip(outputs(code, base[which], code is turbo), outputs(code, base, code is turbo)):
             assert np.array_equal(got, want[which])
+
+
+@pytest.mark.parametrize("constituents", [1, 2])
+@pytest.mark.parametrize("frames", [1, 5000])
+def test_a_code_of_no_bits_decodes_to_none(constituents, frames):
+    """A truncated code of no message bits has no trellis steps, inputs or outputs: decode of
+    any number of its frames does nothing, and says so."""
+    import ctypes as C
+    import fecl_b200 as F
+    from fecl_b200 import _lib
+    code = F.Turbo(F.Turbo.EncoderOptions([F.Trellis(*T17)], [np.zeros(0, np.uint32)] * constituents).termination(1),
+                   F.Turbo.DecoderOptions().algorithm(F.Linear).iterations(2))
+    assert code.msgSize() == 0 and code.paritySize() == 0
+    llr, msg, its = np.zeros(1, np.float32), np.full(1, 7, np.uint8), np.zeros(frames, np.int32)
+    assert _lib.lib.fecl_decode(code._h, llr.ctypes.data_as(C.c_void_p), _lib.F32, frames, msg.ctypes.data_as(C.c_void_p),
+                                its.ctypes.data_as(C.c_void_p), _lib.HOST_MEMORY, None) == _lib.OK
+    assert msg[0] == 7 and np.all(its == 2)
